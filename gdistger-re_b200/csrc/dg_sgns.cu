@@ -1572,6 +1572,7 @@ static int train_walks(dg_sgns *s, const dgs::WalkSet &ws, float alpha, dg_train
     a.window = s->p.window;
     a.negative = s->p.negative;
     a.d = s->p.size;
+    a.used = s->out_size;
     a.alpha = alpha > 0 ? alpha : s->p.alpha;
     a.seed_lo = (uint32_t)s->p.seed;
     a.seed_hi = (uint32_t)(s->p.seed >> 32);

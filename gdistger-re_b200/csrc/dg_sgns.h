@@ -81,6 +81,7 @@ struct SgnsArgs {
     uint64_t train_words;
     uint32_t vocab_size;
     int window, negative, d;
+    int used;                           // columns of a row that are not padding (<= d)
     float alpha;
     uint32_t pass, seed_lo, seed_hi;
     int deterministic;
@@ -123,6 +124,9 @@ bool bf_staging_safe(const std::vector<uint32_t> &cn, uint32_t n_master, int neg
 int launch_minibatch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
 // cbow_kernel and __sgNegReuse semantics (dg_sgns_w2v.cu).
 int launch_cbow(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
+// The Hogwild form of CBOW that trains two centres at a time (dg_sgns_cbow.cu) and what it takes.
+bool cbow_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
+int launch_cbow_pair(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
 int launch_plain_hs(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
 // word2vec's Huffman coding (CreateBinaryTree, word2vec.cu:684-740) of counts in
 // vocabulary order, laid out as off[n + 1] / point / code.  false if a code

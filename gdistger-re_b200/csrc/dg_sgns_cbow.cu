@@ -1,0 +1,323 @@
+// Hogwild CBOW on FP32 rows (cbow_kernel, word2vec.cu:401-509), two centres at a
+// time: the form of DG_SGNS_CBOW that trains walks of at most 32 tokens
+// (sgns_cbow_kernel, dg_sgns_w2v.cu, trains longer ones, rows of 512, more than
+// eight negatives and the one-warp deterministic runs).
+//
+// What bounds the rule is the L2's reduction rate.  A centre with cw contexts and
+// n negatives reads cw + 1 + n rows and adds to as many; on rows that L2 holds, a
+// B200 reads 18.1 TB/s of 512-byte rows but reduces into them at 5.9 TB/s (a
+// vector atomic and a bulk reduction alike), and the two times add up: 9 contexts
+// and 6 targets cost 15 x 512 B x (1 / 18.1 + 1 / 5.9) = 1.7 ns a centre, which was
+// the time of the kernel that trains one centre at a time (1.75 ns a token).  The
+// windows of two neighbouring centres are nearly the same rows, so here a warp
+// reads the rows of both at once and each row receives the sum of both centres'
+// e in one atomic: 6 row reads and reductions a centre for the contexts, not 9.
+//
+// Measured on a B200, size 128, window 10, negative 5: a YouTube-shaped round
+// (25.0M tokens) in 33.0 ms instead of 43.8; a round of the 10,000-vertex graph
+// at size 100, whose padding columns are no longer moved, in 0.38 ms instead of
+// 0.54.  What bounds it now: the same L2 reductions (12 rows a centre, 1.36 ns of
+// 1.32 ns a token), then DRAM (5 KB a token, 0.76 ns).
+//
+// Larger groups would save more (four centres: 8.06 ms for 300,000 walks, two:
+// 9.3), but a Hogwild run's rows depend on how many updates are under way unseen
+// and on how many walks are trained at once: with one of the two doubled or
+// halved, the rows of a 10,000-vertex round end 3 to 4 times further from the
+// one-centre kernel's than two equal runs of that kernel from each other.  So
+// 16 warps of an SM train two centres each, where sgns_cbow_kernel's 32 train
+// one, and each holds two walks that it trains in turn: 32 walks, 32 centres
+// under way (8 of each at 256 columns, where a warp holds one walk and eight
+// warps fit).  The rows then differ 1.4 to 1.7 times as far as two equal runs.
+#include "dg_sgns.h"
+#include "dg_sgns_dev.cuh"
+
+#include <algorithm>
+
+namespace dgs {
+
+constexpr int kCbowWarps = 8;             // warps of a block
+constexpr uint32_t kCbowMaxTokens = 32;   // a lane per token
+constexpr int kCbowFixedNeg = 5;
+constexpr int kCbowPairNeg = 8;           // the largest negative count of this kernel
+
+constexpr int cbow_pair_walks(int vec) { return vec <= 4 ? 2 : 1; }    // walks that a warp trains in turn
+constexpr int cbow_pair_blocks(int vec) { return vec <= 4 ? 2 : 1; }   // blocks per SM
+
+// A walk under way: its length, its next centre, and for token / centre `lane` the
+// word, the positions that hold the same word, the window as a mask of positions
+// and the targets' flags (bit j: target j trains, 0 being the centre's word; bit
+// 31: a target repeats).
+struct CbowWalk {
+    uint32_t n = 0, p = 0;
+    int32_t word = 0;
+    uint32_t same = 0, win = 0, flags = 0;
+    int32_t *sen = nullptr, *negs = nullptr;   // shared: the words, the negatives of every centre
+};
+
+// Lane l owns columns [l * VEC, l * VEC + VEC) of every row and, beside that, token
+// l of the walk (CbowWalk).  A warp holds `walks` walks and trains two centres of
+// each in turn.
+//
+// The second centre's context rows were read before the first centre's e: they
+// are short of it by e times the number of (position of one window, position of
+// the other) pairs that hold one word, which is added to their sum.  So this
+// warp's own updates are all seen.  Target rows are read when their centre
+// starts, after the reductions of the centre before.
+//
+// NS: the negatives at compile time (5), or up to 8 read from a.negative.
+template <int VEC, int NS, bool HS>
+__global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
+    sgns_cbow_pair_kernel(SgnsArgs a, WalkSet ws, uint32_t walks) {
+    constexpr int D = 32 * VEC, M = pow2_at_least(NS + 1), GROUP = 32 / M;
+    constexpr int BATCH = VEC <= 4 ? 8 : 4;   // context rows in flight together
+    constexpr uint32_t kAll = 0xffffffffu;
+    __shared__ __align__(16) int32_t sen_all[kCbowWarps][2][kCbowMaxTokens];
+    __shared__ int32_t negs_all[kCbowWarps][2][kCbowMaxTokens * NS];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int neg = NS == kCbowFixedNeg ? kCbowFixedNeg : a.negative;
+    const uint32_t w = (uint32_t)a.window;
+    // Lanes whose columns are all padding (a size such as 100 or 200, stored with
+    // the next power of two) read lane 0's columns, hold x = 0 and write nothing.
+    const bool own = lane * VEC < (uint32_t)a.used;
+    float *const syn0 = a.syn0 + (own ? lane * VEC : 0), *const syn1 = a.syn1 + (own ? lane * VEC : 0);
+    unsigned long long n_words = 0, n_trained = 0, n_pairs = 0;
+    CbowWalk A, B;
+    A.sen = sen_all[warp][0];
+    A.negs = negs_all[warp][0];
+    B.sen = sen_all[warp][1];
+    B.negs = negs_all[warp][1];
+    bool more = true;
+
+    // The next walk of at least two tokens into A; A.n = 0 when there is none left.
+    auto fetch = [&]() {
+        A.n = A.p = 0;
+        while (more) {
+            uint32_t walk = 0;
+            if (lane == 0) walk = atomicAdd(a.queue, 1u);
+            walk = __shfl_sync(kAll, walk, 0);
+            more = walk < ws.n_walks;
+            if (!more) return;
+            const uint32_t wid = ws.ids ? ws.ids[walk] : walk + ws.id_base;
+            uint32_t words;
+            __syncwarp();
+            const uint32_t n = warp_sentence<kCbowMaxTokens>(ws, walk, a, A.sen, words);
+            n_words += words;
+            n_trained += n;
+            if (n < 2) continue;
+            A.n = n;
+            A.word = lane < n ? A.sen[lane] : -1 - (int32_t)lane;
+            A.same = __match_any_sync(kAll, A.word);
+            A.win = 0;
+            if (lane < n) {   // positions within the shrunk span, the centre excluded
+                const uint32_t span = w - philox(lane, wid, a.pass, kWinTag, a.seed_lo, a.seed_hi).x % w;
+                const uint32_t lo = lane > span ? lane - span : 0u, hi = min(n - 1, lane + span);
+                A.win = ((kAll >> (31 - (hi - lo))) << lo) & ~(1u << lane);
+                n_pairs += __popc(A.win);
+            }
+            for (uint32_t q = lane; q < n * (uint32_t)neg; q += 32) {
+                const uint32_t p = q / (uint32_t)neg, j = q % (uint32_t)neg;
+                A.negs[p * NS + j] = tagged_negative(a, p, wid, kCbowTag, (int)j);
+            }
+            __syncwarp();
+            A.flags = 1;
+            if (lane < n)
+                for (int j = 0; j < neg; j++) {
+                    const int32_t t = A.negs[lane * NS + j];
+                    if (t == A.word) continue;
+                    A.flags |= 2u << j;
+                    for (int i = 0; i < j; i++)
+                        if (A.negs[lane * NS + i] == t) A.flags |= 0x80000000u;
+                }
+            return;
+        }
+    };
+    // The target rows of centre p (a target that does not train reads the centre's row, unused).
+    struct Targets {
+        int32_t t[NS + 1];
+        RowVec<VEC> row[NS + 1];
+    };
+    auto load_targets = [&](uint32_t p, Targets &q) {
+        q.t[0] = A.sen[p];
+#pragma unroll
+        for (int j = 0; j < NS; j++) q.t[j + 1] = j < neg ? A.negs[p * NS + j] : q.t[0];
+#pragma unroll
+        for (int j = 0; j <= NS; j++)
+            if (j <= neg) load_row<VEC>(syn1 + (size_t)q.t[j] * D, q.row[j]);
+    };
+    // The target rows of centre p of walk W on their way to L2, a lane per row.
+    auto prefetch_targets = [&](const CbowWalk &W, uint32_t p) {
+        if (p >= W.n || (int)lane > neg) return;
+        const int32_t t = lane == 0 ? W.sen[p] : W.negs[p * NS + lane - 1];
+        prefetch_l2(a.syn1 + (size_t)t * D, D * 4);
+    };
+    // Centre p's targets against x, the mean of its context rows: e receives the
+    // gradient of x, the target rows their updates (word2vec.cu:453-497).
+    auto train_targets = [&](uint32_t p, const RowVec<VEC> &x, RowVec<VEC> &e, Targets &q) {
+        const uint32_t fl = __shfl_sync(kAll, A.flags, p);
+        if (!(fl & 0x80000000u)) {   // all sums and gradients at once
+            float f[M];
+#pragma unroll
+            for (int j = 0; j < M; j++) f[j] = j <= NS && j <= neg ? row_dot(x, q.row[j <= NS ? j : 0]) : 0.f;
+            const float mine = warp_sums_split<M>(f, lane);
+            const uint32_t jm = lane / GROUP;
+            const float gm = (fl >> jm) & 1u ? sg_grad(mine, jm == 0, a.exp_table, a.alpha) : 0.f;
+#pragma unroll
+            for (int j = 0; j <= NS; j++) {
+                const float g = __shfl_sync(kAll, gm, j * GROUP);
+                if (!((fl >> j) & 1u)) continue;
+                row_fma(e, g, q.row[j]);
+                if (own) add_row<VEC>(syn1 + (size_t)q.t[j] * D, row_mul(g, x));
+            }
+        } else {   // a target repeats: one after the other, each seeing the updates before it
+#pragma unroll
+            for (int j = 0; j <= NS; j++) {
+                if (!((fl >> j) & 1u)) continue;
+                const float g = sg_grad(warp_dot<VEC>(x, q.row[j]), j == 0, a.exp_table, a.alpha);
+                row_fma(e, g, q.row[j]);
+                const RowVec<VEC> upd = row_mul(g, x);
+                row_add(q.row[j], upd);
+                if (own) add_row<VEC>(syn1 + (size_t)q.t[j] * D, upd);
+#pragma unroll
+                for (int k = j + 1; k <= NS; k++)
+                    if (q.t[k] == q.t[j]) q.row[k] = q.row[j];
+            }
+        }
+    };
+    // x / cw, correctly rounded from the rounded reciprocal (Markstein 1990):
+    // q = x r, then q + (x - q cw) r.  Padding lanes become 0.
+    auto mean = [&](RowVec<VEC> &x, uint32_t window) {
+        const float cw = (float)__popc(window), r = __frcp_rn(cw);
+#pragma unroll
+        for (int i = 0; i < VEC; i++) {
+            const float q = x.v[i] * r;
+            x.v[i] = own ? fmaf(fmaf(-q, cw, x.v[i]), r, q) : 0.f;
+        }
+    };
+
+    for (;;) {
+        if (A.p >= A.n) {
+            fetch();
+            if (A.n == 0 && B.p >= B.n) break;
+        }
+        if (A.n) {
+            const uint32_t p = A.p;
+            const uint32_t wp = __shfl_sync(kAll, A.win, p);
+            const uint32_t wq = p + 1 < A.n ? __shfl_sync(kAll, A.win, (p + 1) & 31) : 0u;
+            const uint32_t all = wp | wq, b0 = ((uint32_t)__ffs(all) - 1) & ~3u;
+            prefetch_targets(A, p + 1);
+            prefetch_targets(B, B.p);
+            Targets q;
+            if (!HS) load_targets(p, q);
+            // Context rows of both centres, summed in window order (word2vec.cu:419-428).
+            RowVec<VEC> x, y, e;
+            zero_row(x);
+            zero_row(y);
+            for (uint32_t b = b0; b < 32 && (all >> b); b += BATCH) {
+                RowVec<VEC> r[BATCH];
+#pragma unroll
+                for (int h = 0; h < BATCH; h += 4) {
+                    if (b + h >= 32) break;
+                    const int4 c = *reinterpret_cast<const int4 *>(A.sen + b + h);
+                    const int32_t id[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if ((all >> (b + h + k)) & 1u) load_row<VEC>(syn0 + (size_t)id[k] * D, r[h + k]);
+                }
+#pragma unroll
+                for (int k = 0; k < BATCH; k++) {
+                    if (b + k >= 32) break;
+                    if ((wp >> (b + k)) & 1u) row_add(x, r[k]);
+                    if ((wq >> (b + k)) & 1u) row_add(y, r[k]);
+                }
+            }
+            mean(x, wp);
+            zero_row(e);
+            if (HS) {
+                hs_path<VEC>(a, A.sen[p], x, e, lane);
+                load_targets(p, q);
+            }
+            train_targets(p, x, e, q);
+            if (wq) {
+                if (!HS) load_targets(p + 1, q);
+                const int pairs = __reduce_add_sync(kAll, ((wq >> lane) & 1u) ? __popc(A.same & wp) : 0);
+                row_fma(y, (float)pairs, e);
+                mean(y, wq);
+                zero_row(x);   // from here the second centre's e
+                if (HS) {
+                    hs_path<VEC>(a, A.sen[p + 1], y, x, lane);
+                    load_targets(p + 1, q);
+                }
+                train_targets(p + 1, y, x, q);
+            }
+            // e to every context row (word2vec.cu:498-505), both centres' at once.
+            for (uint32_t b = b0; b < 32 && (all >> b); b += 4) {
+                const int4 c = *reinterpret_cast<const int4 *>(A.sen + b);
+                const int32_t id[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (!((all >> (b + k)) & 1u)) continue;
+                    RowVec<VEC> s;
+                    zero_row(s);
+                    if ((wp >> (b + k)) & 1u) s = e;
+                    if ((wq >> (b + k)) & 1u) row_add(s, x);
+                    if (own) add_row<VEC>(syn0 + (size_t)id[k] * D, s);
+                }
+            }
+            A.p = p + 2;
+        }
+        if (walks > 1) {
+            const CbowWalk t = A;
+            A = B;
+            B = t;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) n_pairs += __shfl_xor_sync(kAll, n_pairs, o);
+    if (lane == 0) {
+        atomicAdd(&a.stats[0], n_words);
+        atomicAdd(&a.stats[1], n_trained);
+        atomicAdd(&a.stats[2], n_pairs);
+    }
+}
+
+bool cbow_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    return s->p.mode == DG_SGNS_CBOW && !s->p.deterministic && ws.max_len > 0 && ws.max_len <= kCbowMaxTokens &&
+           s->p.size <= 256 && a.negative <= kCbowPairNeg && a.vocab_size > 1;
+}
+
+template <int V, int NS, bool HS>
+static int cbow_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    auto kern = sgns_cbow_pair_kernel<V, NS, HS>;
+    const uint32_t want = s->p.workers;   // the caller's bound on walks under way: a warp each, or two if need be
+    const int warps = want > 0 && want < (uint32_t)kCbowWarps ? (int)want : kCbowWarps;
+    int per_sm = 0;
+    DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, 0));
+    int blocks = std::min(std::max(per_sm, 1), cbow_pair_blocks(V)) * dg::sm_count(s->device);
+    const uint32_t walks = want > 0 && want <= (uint32_t)(blocks * warps) ? 1u : (uint32_t)cbow_pair_walks(V);
+    if (want > 0) blocks = std::min(blocks, std::max(1, (int)(want / (walks * (uint32_t)warps))));
+    kern<<<blocks, 32 * warps, 0, s->stream>>>(a, ws, walks);
+    dg::note_launch();
+    DG_CUDA(cudaGetLastError());
+    return DG_OK;
+}
+
+template <int V>
+static int cbow_pair_size(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    const bool fixed = a.negative == kCbowFixedNeg;
+    if (a.hs)
+        return fixed ? cbow_pair_launch<V, kCbowFixedNeg, true>(s, a, ws)
+                     : cbow_pair_launch<V, kCbowPairNeg, true>(s, a, ws);
+    return fixed ? cbow_pair_launch<V, kCbowFixedNeg, false>(s, a, ws)
+                 : cbow_pair_launch<V, kCbowPairNeg, false>(s, a, ws);
+}
+
+int launch_cbow_pair(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    switch (s->p.size / 32) {
+    case 1: return cbow_pair_size<1>(s, a, ws);
+    case 2: return cbow_pair_size<2>(s, a, ws);
+    case 4: return cbow_pair_size<4>(s, a, ws);
+    default: return cbow_pair_size<8>(s, a, ws);
+    }
+}
+
+}  // namespace dgs

@@ -68,6 +68,85 @@ __device__ __forceinline__ float warp_dot(const RowVec<VEC> &a, const RowVec<VEC
 }
 
 
+// Packed FP32 pairs (add / mul / fma.rn.f32x2): each half rounds as the scalar
+// operation does, two columns to an instruction.
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long r, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r));
+}
+
+// a += b
+template <int VEC>
+__device__ __forceinline__ void row_add(RowVec<VEC> &a, const RowVec<VEC> &b) {
+    if constexpr (VEC == 1) {
+        a.v[0] += b.v[0];
+    } else {
+#pragma unroll
+        for (int i = 0; i < VEC; i += 2) {
+            unsigned long long r;
+            asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a.v[i], a.v[i + 1])), "l"(pack2(b.v[i], b.v[i + 1])));
+            unpack2(r, a.v[i], a.v[i + 1]);
+        }
+    }
+}
+
+// a += s * b, fused
+template <int VEC>
+__device__ __forceinline__ void row_fma(RowVec<VEC> &a, float s, const RowVec<VEC> &b) {
+    if constexpr (VEC == 1) {
+        a.v[0] = fmaf(s, b.v[0], a.v[0]);
+    } else {
+        const unsigned long long ss = pack2(s, s);
+#pragma unroll
+        for (int i = 0; i < VEC; i += 2) {
+            unsigned long long r;
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r)
+                : "l"(ss), "l"(pack2(b.v[i], b.v[i + 1])), "l"(pack2(a.v[i], a.v[i + 1])));
+            unpack2(r, a.v[i], a.v[i + 1]);
+        }
+    }
+}
+
+// s * b, rounded
+template <int VEC>
+__device__ __forceinline__ RowVec<VEC> row_mul(float s, const RowVec<VEC> &b) {
+    RowVec<VEC> o;
+    if constexpr (VEC == 1) {
+        o.v[0] = __fmul_rn(s, b.v[0]);
+    } else {
+        const unsigned long long ss = pack2(s, s);
+#pragma unroll
+        for (int i = 0; i < VEC; i += 2) {
+            unsigned long long r;
+            asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(ss), "l"(pack2(b.v[i], b.v[i + 1])));
+            unpack2(r, o.v[i], o.v[i + 1]);
+        }
+    }
+    return o;
+}
+
+// This lane's part of a dot product: even and odd columns in two fused chains.
+template <int VEC>
+__device__ __forceinline__ float row_dot(const RowVec<VEC> &a, const RowVec<VEC> &b) {
+    if constexpr (VEC == 1) {
+        return a.v[0] * b.v[0];
+    } else {
+        unsigned long long r;
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a.v[0], a.v[1])), "l"(pack2(b.v[0], b.v[1])));
+#pragma unroll
+        for (int i = 2; i < VEC; i += 2)
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r)
+                : "l"(pack2(a.v[i], a.v[i + 1])), "l"(pack2(b.v[i], b.v[i + 1])), "l"(r));
+        float lo, hi;
+        unpack2(r, lo, hi);
+        return lo + hi;
+    }
+}
+
 // g = (label - sigmoid(f)) * alpha through expTable (word2vec.cu:383-388), with
 // the reference's integer-division index scale (EXP_TABLE_SIZE / MAX_EXP / 2 = 83).
 __device__ __forceinline__ float sg_grad(float f, int label, const float *exp_table, float alpha) {
@@ -117,6 +196,56 @@ __device__ __forceinline__ uint32_t warp_sentence(const WalkSet &ws, uint32_t wa
     }
     __syncwarp();
     return n;
+}
+
+// ------------------------------------------------ word2vec rules
+
+// Negative j (0-based) drawn from (c0, walk, pass, tag + j/4), word j%4, with
+// word2vec's replacement of index 0 (word2vec.cu:365-368).
+__device__ __forceinline__ int32_t tagged_negative(const SgnsArgs &a, uint32_t c0, uint32_t wid, uint32_t tag, int j) {
+    const uint4 blk = philox(c0, wid, a.pass, tag + (uint32_t)(j >> 2), a.seed_lo, a.seed_hi);
+    const uint32_t q = j & 3;
+    const uint32_t r = q == 0 ? blk.x : q == 1 ? blk.y : q == 2 ? blk.z : blk.w;
+    int32_t t = a.table[r % a.table_size];
+    if (t == 0) t = (int32_t)((r >> 8) % (a.vocab_size - 1) + 1);
+    return t;
+}
+
+template <int VEC>
+__device__ __forceinline__ void zero_row(RowVec<VEC> &r) {
+#pragma unroll
+    for (int i = 0; i < VEC; i++) r.v[i] = 0.f;
+}
+
+// Hierarchical softmax over the Huffman path of `word` (word2vec.cu:334-356,
+// 436-455): per inner node, f = x . syn1[node]; nodes with |f| >= MAX_EXP are
+// skipped, else g = (1 - code - sigmoid(f)) alpha, e += g syn1[node] (fused),
+// syn1[node] += rounded g x.  Inner nodes index the same output table as the
+// words, so every node row is read before and written after its own update.
+template <int VEC>
+__device__ __forceinline__ void hs_path(const SgnsArgs &a, int32_t word, const RowVec<VEC> &x, RowVec<VEC> &e,
+                                        uint32_t lane) {
+    const int d = 32 * VEC;
+    const int32_t k0 = a.hs_off[word], k1 = a.hs_off[word + 1];
+    for (int32_t k = k0; k < k1; k++) {
+        float *rp = a.syn1 + (size_t)a.hs_point[k] * d + lane * VEC;
+        RowVec<VEC> row;
+        load_row<VEC>(rp, row);
+        const float f = warp_dot<VEC>(x, row);
+        if (f <= -kMaxExp || f >= kMaxExp) continue;
+        const float g =
+            ((float)(1 - a.hs_code[k]) - __ldg(a.exp_table + (int)((f + kMaxExp) * (kExpTableSize / kMaxExp / 2)))) *
+            a.alpha;
+        RowVec<VEC> upd;
+#pragma unroll
+        for (int i = 0; i < VEC; i++) {
+            e.v[i] = fmaf(g, row.v[i], e.v[i]);
+            upd.v[i] = __fmul_rn(g, x.v[i]);
+            row.v[i] += upd.v[i];
+        }
+        if (a.deterministic) store_row<VEC>(rp, row);
+        else add_row<VEC>(rp, upd);
+    }
 }
 
 // ------------------------------------------------------------ BF16 rows

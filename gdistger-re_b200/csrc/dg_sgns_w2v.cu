@@ -28,54 +28,6 @@ namespace dgs {
 
 constexpr int kW2vThreads = 256;
 
-// Negative j (0-based) drawn from (c0, walk, pass, tag + j/4), word j%4, with
-// word2vec's replacement of index 0 (word2vec.cu:365-368).
-__device__ __forceinline__ int32_t tagged_negative(const SgnsArgs &a, uint32_t c0, uint32_t wid, uint32_t tag, int j) {
-    const uint4 blk = philox(c0, wid, a.pass, tag + (uint32_t)(j >> 2), a.seed_lo, a.seed_hi);
-    const uint32_t q = j & 3;
-    const uint32_t r = q == 0 ? blk.x : q == 1 ? blk.y : q == 2 ? blk.z : blk.w;
-    int32_t t = a.table[r % a.table_size];
-    if (t == 0) t = (int32_t)((r >> 8) % (a.vocab_size - 1) + 1);
-    return t;
-}
-
-template <int VEC>
-__device__ __forceinline__ void zero_row(RowVec<VEC> &r) {
-#pragma unroll
-    for (int i = 0; i < VEC; i++) r.v[i] = 0.f;
-}
-
-// Hierarchical softmax over the Huffman path of `word` (word2vec.cu:334-356,
-// 436-455): per inner node, f = x . syn1[node]; nodes with |f| >= MAX_EXP are
-// skipped, else g = (1 - code - sigmoid(f)) alpha, e += g syn1[node] (fused),
-// syn1[node] += rounded g x.  Inner nodes index the same output table as the
-// words, so every node row is read before and written after its own update.
-template <int VEC>
-__device__ __forceinline__ void hs_path(const SgnsArgs &a, int32_t word, const RowVec<VEC> &x, RowVec<VEC> &e,
-                                        uint32_t lane) {
-    const int d = 32 * VEC;
-    const int32_t k0 = a.hs_off[word], k1 = a.hs_off[word + 1];
-    for (int32_t k = k0; k < k1; k++) {
-        float *rp = a.syn1 + (size_t)a.hs_point[k] * d + lane * VEC;
-        RowVec<VEC> row;
-        load_row<VEC>(rp, row);
-        const float f = warp_dot<VEC>(x, row);
-        if (f <= -kMaxExp || f >= kMaxExp) continue;
-        const float g =
-            ((float)(1 - a.hs_code[k]) - __ldg(a.exp_table + (int)((f + kMaxExp) * (kExpTableSize / kMaxExp / 2)))) *
-            a.alpha;
-        RowVec<VEC> upd;
-#pragma unroll
-        for (int i = 0; i < VEC; i++) {
-            e.v[i] = fmaf(g, row.v[i], e.v[i]);
-            upd.v[i] = __fmul_rn(g, x.v[i]);
-            row.v[i] += upd.v[i];
-        }
-        if (a.deterministic) store_row<VEC>(rp, row);
-        else add_row<VEC>(rp, upd);
-    }
-}
-
 // ------------------------------------------------------------------ CBOW
 
 // Blocks per SM the CBOW kernel's registers are capped for: the kernel waits on
@@ -469,6 +421,7 @@ static int negshare_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
 }
 
 int launch_cbow(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    if (cbow_pair_applies(s, a, ws)) return launch_cbow_pair(s, a, ws);
     if (s->p.mode == DG_SGNS_CBOW_BF16) {
         switch (s->p.size / 32) {
             case 2: return cbow_launch<2, true>(s, a, ws);

@@ -134,6 +134,9 @@ int launch_plain_hs(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
 bool huffman_codes(const std::vector<uint32_t> &cn, std::vector<int32_t> &off, std::vector<int32_t> &point,
                    std::vector<int8_t> &code);
 int launch_negshare(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
+// The Hogwild form of the shared-negative rule that trains two pairs at a time (dg_sgns_negshare.cu) and what it takes.
+bool negshare_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
+int launch_negshare_pair(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
 constexpr int kCbowMaxNeg = 32;   // one negative per lane
 constexpr int kShareMaxNeg = 16;  // shared negatives held in shared memory per warp
 

@@ -1,0 +1,251 @@
+// Hogwild shared-negative skip-gram on FP32 rows (__sgNegReuse, word2vec.cu:231-303),
+// two pairs at a time: the form of DG_SGNS_SG_SHARED that trains walks of at most
+// 64 tokens with rows of 64 to 256 columns and up to eight negatives
+// (sgns_negshare_kernel, dg_sgns_w2v.cu, trains the others and the deterministic
+// runs).
+//
+// What bounds the rule is the L2's reduction rate (5.9 TB/s of 512-byte rows on a
+// B200, against 18.1 TB/s of reads; the two times add up): a walk's negatives stay
+// in L2, and each pair read and updated n + 1 rows there.  A walk's pairs share
+// the negatives, so here a warp reads them once for two pairs of a centre, lets
+// the second pair see the first one's update in registers, and sends the sum of
+// both: n + 2 rows for two pairs instead of 2 n + 2.  Padding columns (size 200 in
+// rows of 256) are not moved.
+//
+// A Hogwild run's rows depend on how many pairs are under way unseen and on how
+// many walks are trained at once (dg_sgns_cbow.cu), so half as many warps as
+// sgns_negshare_kernel's hold two walks each and train a centre of either in turn.
+//
+// A round of the 50,000-vertex graph at size 200, window 5, negative 5, with its
+// read-back: 20.5 -> 12.6 ms.  The rows end 1.3 to 2 times as far from the one-pair
+// kernel's as two equal runs of that kernel from each other.
+#include "dg_sgns.h"
+#include "dg_sgns_dev.cuh"
+
+#include <algorithm>
+
+namespace dgs {
+
+constexpr int kShareWarps = 8;             // warps of a block
+constexpr uint32_t kShareTokens = 64;      // the longest walk of this kernel
+constexpr int kShareFixedNeg = 5;
+constexpr int kSharePairNeg = 8;           // the largest negative count of this kernel
+
+// Blocks per SM: two walks a warp, 32 walks up to 128 columns, 16 at 256.
+constexpr int share_pair_blocks(int vec) { return vec <= 4 ? 2 : 1; }
+
+// A walk under way: its length and next centre, its words and negatives (shared),
+// and whether a negative occurs twice.
+struct ShareWalk {
+    uint32_t n = 0, p = 0;
+    int32_t *sen = nullptr, *negs = nullptr;
+    bool repeat = false;
+};
+
+// Lane l owns columns [l * VEC, l * VEC + VEC) of every row.  NS: the negatives at
+// compile time (5), or up to 8 read from a.negative.
+template <int VEC, int NS>
+__global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
+    sgns_negshare_pair_kernel(SgnsArgs a, WalkSet ws, uint32_t walks) {
+    constexpr int D = 32 * VEC, M = pow2_at_least(NS + 1), GROUP = 32 / M;
+    constexpr uint32_t kAll = 0xffffffffu;
+    __shared__ int32_t sen_all[kShareWarps][2][kShareTokens];
+    __shared__ int32_t negs_all[kShareWarps][2][NS];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int neg = NS == kShareFixedNeg ? kShareFixedNeg : a.negative;
+    const uint32_t w = (uint32_t)a.window;
+    // Lanes whose columns are all padding read lane 0's columns, hold context rows of 0 and write nothing.
+    const bool own = lane * VEC < (uint32_t)a.used;
+    float *const syn0 = a.syn0 + (own ? lane * VEC : 0), *const syn1 = a.syn1 + (own ? lane * VEC : 0);
+    unsigned long long n_words = 0, n_trained = 0, n_pairs = 0;
+    ShareWalk A, B;
+    A.sen = sen_all[warp][0];
+    A.negs = negs_all[warp][0];
+    B.sen = sen_all[warp][1];
+    B.negs = negs_all[warp][1];
+    bool more = true;
+
+    auto fetch = [&]() {   // the next walk of at least two tokens into A; A.n = 0 when there is none left
+        A.n = A.p = 0;
+        while (more) {
+            uint32_t walk = 0;
+            if (lane == 0) walk = atomicAdd(a.queue, 1u);
+            walk = __shfl_sync(kAll, walk, 0);
+            more = walk < ws.n_walks;
+            if (!more) return;
+            const uint32_t wid = ws.ids ? ws.ids[walk] : walk + ws.id_base;
+            uint32_t words;
+            __syncwarp();
+            const uint32_t n = warp_sentence<kShareTokens>(ws, walk, a, A.sen, words);
+            n_words += words;
+            n_trained += n;
+            if (n < 2) continue;
+            A.n = n;
+            int32_t t = -1 - (int32_t)lane;
+            if ((int)lane < neg) A.negs[lane] = t = tagged_negative(a, 0, wid, kShareTag, (int)lane);
+            const uint32_t same = __match_any_sync(kAll, t);
+            A.repeat = __any_sync(kAll, (same & (same - 1)) != 0u);
+            __syncwarp();
+            return;
+        }
+    };
+    auto load_context = [&](int32_t word, RowVec<VEC> &r) {
+        load_row<VEC>(syn0 + (size_t)word * D, r);
+        if (!own) zero_row(r);
+    };
+
+    for (;;) {
+        if (A.p >= A.n) {
+            fetch();
+            if (A.n == 0 && B.p >= B.n) break;
+        }
+        if (A.n) {
+            const uint32_t p = A.p, n = A.n;
+            const int32_t word = A.sen[p];
+            RowVec<VEC> pos, pos0;
+            load_row<VEC>(syn1 + (size_t)word * D, pos);
+            pos0 = pos;
+            int32_t t[NS];
+            uint32_t live = 0;   // bit j: negative j trains (it is not the centre's word)
+#pragma unroll
+            for (int j = 0; j < NS; j++) {
+                t[j] = j < neg ? A.negs[j] : word;
+                if (j < neg && t[j] != word) live |= 1u << j;
+            }
+            const uint32_t lo = p > w ? p - w : 0u, hi = min(n, p + w + 1);   // positions; p itself is no context
+            const uint32_t m = hi - lo - 1;
+            n_pairs += m;
+            auto at = [&](uint32_t k) { return A.sen[lo + k + (lo + k >= p ? 1u : 0u)]; };
+            // The gradients of the pair (l, centre): lane group j holds negative j's, group neg's the
+            // positive's; all sums are of the rows as they are.
+            auto gradients = [&](const RowVec<VEC> &l, const RowVec<VEC> (&row)[NS]) {
+                float f[M];
+#pragma unroll
+                for (int j = 0; j < M; j++) f[j] = j < NS ? row_dot(l, row[j < NS ? j : 0]) : j == NS ? row_dot(l, pos) : 0.f;
+                const float mine = warp_sums_split<M>(f, lane);
+                const uint32_t jm = lane / GROUP;
+                float g = 0.f;
+                if (jm == (uint32_t)NS || ((live >> jm) & 1u)) g = sg_grad(mine, jm == (uint32_t)NS, a.exp_table, a.alpha);
+                return g;
+            };
+            if (!A.repeat) {
+                for (uint32_t k = 0; k < m; k += 2) {
+                    const bool two = k + 1 < m;
+                    const int32_t w1 = at(k), w2 = two ? at(k + 1) : w1;
+                    RowVec<VEC> l1, l2, e, row[NS];
+                    load_context(w1, l1);
+                    load_context(w2, l2);
+#pragma unroll
+                    for (int j = 0; j < NS; j++)
+                        if (j < neg) load_row<VEC>(syn1 + (size_t)t[j] * D, row[j]);
+                        else zero_row(row[j]);
+                    const float ga = gradients(l1, row);
+                    zero_row(e);
+#pragma unroll
+                    for (int j = 0; j < NS; j++) {
+                        const float g = __shfl_sync(kAll, ga, j * GROUP);   // 0 where the negative does not train
+                        row_fma(e, g, row[j]);
+                        if (two) row_fma(row[j], g, l1);
+                    }
+                    {
+                        const float g = __shfl_sync(kAll, ga, NS * GROUP);
+                        row_fma(e, g, pos);
+                        row_fma(pos, g, l1);
+                    }
+                    if (own) add_row<VEC>(syn0 + (size_t)w1 * D, e);
+                    float gb = 0.f;
+                    if (two) {
+                        if (w2 == w1) row_add(l2, e);   // one word twice: the second pair sees the first one's update
+                        gb = gradients(l2, row);
+                        zero_row(e);
+#pragma unroll
+                        for (int j = 0; j < NS; j++) row_fma(e, __shfl_sync(kAll, gb, j * GROUP), row[j]);
+                        const float g = __shfl_sync(kAll, gb, NS * GROUP);
+                        row_fma(e, g, pos);
+                        row_fma(pos, g, l2);
+                        if (own) add_row<VEC>(syn0 + (size_t)w2 * D, e);
+                    }
+#pragma unroll
+                    for (int j = 0; j < NS; j++) {
+                        const float g1 = __shfl_sync(kAll, ga, j * GROUP), g2 = __shfl_sync(kAll, gb, j * GROUP);
+                        if (!((live >> j) & 1u)) continue;
+                        RowVec<VEC> upd = row_mul(g1, l1);
+                        row_fma(upd, g2, l2);
+                        if (own) add_row<VEC>(syn1 + (size_t)t[j] * D, upd);
+                    }
+                }
+            } else {   // a negative occurs twice: one target after the other
+                for (uint32_t k = 0; k < m; k++) {
+                    const int32_t w1 = at(k);
+                    RowVec<VEC> l1, e;
+                    load_context(w1, l1);
+                    zero_row(e);
+                    for (int j = 0; j < neg; j++) {
+                        const int32_t tj = A.negs[j];
+                        if (tj == word) continue;
+                        RowVec<VEC> row;
+                        load_row<VEC>(syn1 + (size_t)tj * D, row);
+                        const float g = sg_grad(warp_dot<VEC>(l1, row), 0, a.exp_table, a.alpha);
+                        row_fma(e, g, row);
+                        if (own) add_row<VEC>(syn1 + (size_t)tj * D, row_mul(g, l1));
+                    }
+                    const float g = sg_grad(warp_dot<VEC>(l1, pos), 1, a.exp_table, a.alpha);
+                    row_fma(e, g, pos);
+                    row_fma(pos, g, l1);
+                    if (own) add_row<VEC>(syn0 + (size_t)w1 * D, e);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < VEC; i++) pos.v[i] -= pos0.v[i];
+            if (own) add_row<VEC>(syn1 + (size_t)word * D, pos);
+            A.p = p + 1;
+        }
+        if (walks > 1) {
+            const ShareWalk x = A;
+            A = B;
+            B = x;
+        }
+    }
+    if (lane == 0) {
+        atomicAdd(&a.stats[0], n_words);
+        atomicAdd(&a.stats[1], n_trained);
+        atomicAdd(&a.stats[2], n_pairs);
+    }
+}
+
+bool negshare_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    return !s->p.deterministic && ws.max_len > 0 && ws.max_len <= kShareTokens && s->p.size >= 64 && s->p.size <= 256 &&
+           a.negative <= kSharePairNeg && a.vocab_size > 1;
+}
+
+template <int V, int NS>
+static int negshare_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    auto kern = sgns_negshare_pair_kernel<V, NS>;
+    const uint32_t want = s->p.workers;   // the caller's bound on walks under way: a warp each, or two if need be
+    const int warps = want > 0 && want < (uint32_t)kShareWarps ? (int)want : kShareWarps;
+    int per_sm = 0;
+    DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, 0));
+    int blocks = std::min(std::max(per_sm, 1), share_pair_blocks(V)) * dg::sm_count(s->device);
+    const uint32_t walks = want > 0 && want <= (uint32_t)(blocks * warps) ? 1u : 2u;
+    if (want > 0) blocks = std::min(blocks, std::max(1, (int)(want / (walks * (uint32_t)warps))));
+    kern<<<blocks, 32 * warps, 0, s->stream>>>(a, ws, walks);
+    dg::note_launch();
+    DG_CUDA(cudaGetLastError());
+    return DG_OK;
+}
+
+template <int V>
+static int negshare_pair_size(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    return a.negative == kShareFixedNeg ? negshare_pair_launch<V, kShareFixedNeg>(s, a, ws)
+                                        : negshare_pair_launch<V, kSharePairNeg>(s, a, ws);
+}
+
+int launch_negshare_pair(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    switch (s->p.size / 32) {
+    case 2: return negshare_pair_size<2>(s, a, ws);
+    case 4: return negshare_pair_size<4>(s, a, ws);
+    default: return negshare_pair_size<8>(s, a, ws);
+    }
+}
+
+}  // namespace dgs

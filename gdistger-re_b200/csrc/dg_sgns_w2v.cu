@@ -463,6 +463,7 @@ int launch_plain_hs(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
 }
 
 int launch_negshare(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    if (negshare_pair_applies(s, a, ws)) return launch_negshare_pair(s, a, ws);
     switch (s->p.size / 32) {
         case 1: return negshare_launch<1>(s, a, ws);
         case 2: return negshare_launch<2>(s, a, ws);

@@ -230,7 +230,7 @@ dg_graph::~dg_graph() {
         out_deg.release();
         in_deg.release();
         freq.release();
-        etable.release();
+        etable.release(); step_table.release();
         cudaStreamDestroy(stream);
     }
 }
@@ -243,8 +243,22 @@ int ensure_entropy_table(dg_graph *g, uint32_t max_sn) {
     std::vector<double> t(n);
     for (uint32_t s = 1; s <= max_sn; s++)
         for (uint32_t f = 0; f <= s; f++) t[(uint64_t)s * (s + 1) / 2 + f - 1] = entropy_term((double)s, (double)f);
+    // Step table: entry s is {1 / s in two parts, E(S), E(S^2) - E(S)^2} of a walk of s
+    // footprints (Correlation's recurrences for S, walk.hpp:317-354, from S = 1).
+    std::vector<double4> st((size_t)max_sn + 2);
+    double ES = 1.0, ESS = 1.0;
+    for (uint32_t s = 1; s <= max_sn + 1; s++) {
+        const double S = (double)s, hi = 1.0 / S, lo = std::fma(-hi, S, 1.0) / S;
+        if (s > 1) {
+            ES = ES + (S - ES) / S;
+            ESS = ESS + (S * S - ESS) / S;
+        }
+        st[s] = double4{hi, lo, ES, ESS - ES * ES};
+    }
     DG_CUDA(g->etable.alloc(n));
+    DG_CUDA(g->step_table.alloc(st.size()));
     DG_CUDA(cudaMemcpyAsync(g->etable.p, t.data(), n * 8, cudaMemcpyHostToDevice, g->stream));
+    DG_CUDA(cudaMemcpyAsync(g->step_table.p, st.data(), st.size() * sizeof(double4), cudaMemcpyHostToDevice, g->stream));
     DG_CUDA(cudaStreamSynchronize(g->stream));
     g->etable_max_sn = max_sn;
     return DG_OK;

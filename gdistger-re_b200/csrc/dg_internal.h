@@ -119,6 +119,7 @@ struct dg_graph {
     dg::DevArray<uint32_t> in_deg;    // v_num
     dg::DevArray<uint32_t> freq;      // cumulative visits, v_num
     dg::DevArray<double> etable;      // entropy-term table
+    dg::DevArray<double4> step_table; // what a walk's state shares with every walk of as many footprints
     uint32_t etable_max_sn = 0;
     std::vector<uint32_t> h_out_deg;
     std::vector<double> entropy_history;

@@ -32,6 +32,7 @@ struct WalkArgs {
     const uint64_t *__restrict__ offsets;
     const uint2 *__restrict__ entries;
     const double *__restrict__ etable;
+    const double4 *__restrict__ steps;
     uint32_t *__restrict__ verts;
     uint32_t *__restrict__ lens;
     uint32_t *__restrict__ freq;
@@ -42,31 +43,43 @@ struct WalkArgs {
 };
 
 // Running entropy / effectiveness state of one walk (Correlation, walk.hpp:260-387).
-// N equals S at every step (both start at 1 and grow by 1), so one variable serves both.
+// N equals S at every step (both start at 1 and grow by 1), so one count serves both;
+// and S, E(S) and E(S^2) are the same for every walk after as many steps: they, with
+// the reciprocal of S, come from a table (dg_graph::step_table).  R is formed only
+// where the stop test reads it.
 struct Corr {
-    double S, H, EH, ES, EHS, EHH, ESS, R;
+    double H, EH, EHS, EHH;
 };
 
-// Correlation::iterate with step_k = 1 (walk.hpp:317-354); t = log2 term from the table.
-__device__ __forceinline__ void corr_iterate(Corr &c, double t) {
-    const double S1 = __dadd_rn(c.S, 1.0);
-    const double H1 = __ddiv_rn(__dsub_rn(__dmul_rn(c.S, c.H), t), S1);
-    c.EH = __dadd_rn(c.EH, __ddiv_rn(__dsub_rn(H1, c.EH), S1));
-    c.ES = __dadd_rn(c.ES, __ddiv_rn(__dsub_rn(S1, c.ES), S1));
-    c.EHS = __dadd_rn(c.EHS, __ddiv_rn(__dsub_rn(__dmul_rn(H1, S1), c.EHS), S1));
-    c.EHH = __dadd_rn(c.EHH, __ddiv_rn(__dsub_rn(__dmul_rn(H1, H1), c.EHH), S1));
-    c.ESS = __dadd_rn(c.ESS, __ddiv_rn(__dsub_rn(__dmul_rn(S1, S1), c.ESS), S1));
-    const double DH = __dsub_rn(c.EHH, __dmul_rn(c.EH, c.EH));
-    const double DS = __dsub_rn(c.ESS, __dmul_rn(c.ES, c.ES));
-    const double e = __dsub_rn(c.EHS, __dmul_rn(c.EH, c.ES));
-    c.R = e == 0.0 ? 0.0 : __ddiv_rn(e, __dsqrt_rn(__dmul_rn(DH, DS)));
-    c.H = H1;
-    c.S = S1;
+// a / b correctly rounded, from b's reciprocal in two parts (hi + lo = 1 / b to about
+// 2^-106): q = RN(a hi + RN(a lo)) is within an ulp of a / b, so a - q b is exact and
+// q + (a - q b) hi rounds to a / b (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990).  Here b is a step count and a is neither
+// huge nor subnormal.
+__device__ __forceinline__ double div_by(double a, double b, double hi, double lo) {
+    const double q = __fma_rn(a, hi, __dmul_rn(a, lo));
+    return __fma_rn(__fma_rn(-q, b, a), hi, q);
 }
 
-// walk.hpp:868-872: stop once step > min_len and (R^2 < 0.999 or R < 0).
-__device__ __forceinline__ bool corr_stop(const Corr &c, uint32_t step, uint32_t min_len) {
-    return step > min_len && (__dmul_rn(c.R, c.R) < 0.999 || c.R < 0.0);
+// Correlation::iterate with step_k = 1 (walk.hpp:317-354) for a walk of n footprints so
+// far; t = log2 term from the table, st = the step table's entry of n + 1.
+__device__ __forceinline__ void corr_iterate(Corr &c, double t, uint32_t n, const double4 &st) {
+    const double S = (double)n, S1 = (double)(n + 1);
+    const double H1 = div_by(__dsub_rn(__dmul_rn(S, c.H), t), S1, st.x, st.y);
+    c.EH = __dadd_rn(c.EH, div_by(__dsub_rn(H1, c.EH), S1, st.x, st.y));
+    c.EHS = __dadd_rn(c.EHS, div_by(__dsub_rn(__dmul_rn(H1, S1), c.EHS), S1, st.x, st.y));
+    c.EHH = __dadd_rn(c.EHH, div_by(__dsub_rn(__dmul_rn(H1, H1), c.EHH), S1, st.x, st.y));
+    c.H = H1;
+}
+
+// walk.hpp:868-872: stop once step > min_len and (R^2 < 0.999 or R < 0); st = the step
+// table's entry of the walk's footprints.
+__device__ __forceinline__ bool corr_stop(const Corr &c, uint32_t step, uint32_t min_len, const double4 &st) {
+    if (step <= min_len) return false;
+    const double DH = __dsub_rn(c.EHH, __dmul_rn(c.EH, c.EH));
+    const double e = __dsub_rn(c.EHS, __dmul_rn(c.EH, st.z));
+    const double R = e == 0.0 ? 0.0 : __ddiv_rn(e, __dsqrt_rn(__dmul_rn(DH, st.w)));
+    return __dmul_rn(R, R) < 0.999 || R < 0.0;
 }
 
 __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
@@ -77,15 +90,30 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 
 // Persistent walk kernel: each thread pulls walker ids from a device queue and
 // advances that walk to completion (walk.hpp:845-1024 with every vertex local).
-// Per transition attempt: one Philox block, two loads for the row bounds, one
-// 8-byte CSR entry {neighbour, acceptance threshold}; the accept test is an
-// integer compare.  The walk's footprints go to its arena slot and, for the first
-// kSmemSteps, to a shared-memory copy that serves the prior-visit count
-// (the unordered_map of walk.hpp:816).
+// Per transition attempt: one Philox block, two loads for the row bounds (none after
+// a rejected candidate, which stays on its row), one 8-byte CSR entry {neighbour,
+// acceptance threshold}; the accept test is an integer compare.  The walk's
+// footprints go to its arena slot and, for the first STEPS, to a shared-memory copy
+// that serves the prior-visit count of a candidate (the unordered_map of
+// walk.hpp:816), four footprints to a load; the count of the current vertex, which a
+// rejection steps back to, is carried along.
+//
+// What bounds it is issue slots (64 % of the SM's throughput with the CSR in L2): the
+// FP64 state and the visit counts are most of a footprint, so divisions by the step
+// count go through its tabulated reciprocal, what every walk shares is tabulated, and
+// the next row's bounds are loaded before that arithmetic.  A round of 10,000 walks:
+// 0.049 -> 0.032 ms; of the YouTube-shaped graph (1.14M walks): 0.625 -> 0.485; of the
+// LiveJournal-shaped one (2.24M, a CSR of 242 MB, beyond L2): 1.19 -> 1.15, there
+// the latency of the gathers.
 template <int THREADS, int STEPS>
 __global__ void __launch_bounds__(THREADS) walk_kernel(WalkArgs a) {
-    __shared__ uint32_t cache[STEPS][THREADS];
+    // A thread's footprints are STEPS consecutive words, rows padded by 4: the 16-byte
+    // reads of a quarter warp then hit distinct banks (STEPS a multiple of 8).
+    constexpr int ROW = STEPS + 4;
+    static_assert(STEPS % 8 == 0, "rows of the footprint cache");
+    __shared__ __align__(16) uint32_t cache[THREADS * ROW];
     const int tid = threadIdx.x;
+    uint32_t *const mine = cache + tid * ROW;
     unsigned long long n_fp = 0, n_draw = 0, n_trace = 0, n_over = 0;
     uint32_t longest = 0;
     for (;;) {
@@ -94,28 +122,34 @@ __global__ void __launch_bounds__(THREADS) walk_kernel(WalkArgs a) {
         uint32_t *path = a.verts + (uint64_t)w * a.stride;
         uint32_t cur = w % a.v_num;
         uint32_t n = 0;
+#pragma unroll
+        for (int i = 0; i < STEPS; i += 4)   // no vertex: ids are below v_num
+            *reinterpret_cast<uint4 *>(mine + i) = make_uint4(~0u, ~0u, ~0u, ~0u);
 
-        // Appends v and returns its prior-visit count.
-        auto visit_count = [&](uint32_t v) -> uint32_t {
+        auto visit_count = [&](uint32_t v) -> uint32_t {   // earlier footprints on v
             uint32_t c = 0;
             const uint32_t hot = n < (uint32_t)STEPS ? n : (uint32_t)STEPS;
-            for (uint32_t i = 0; i < hot; i++) c += cache[i][tid] == v;
+            for (uint32_t i = 0; i < hot; i += 4) {
+                const uint4 q = *reinterpret_cast<const uint4 *>(mine + i);
+                c += (q.x == v) + (q.y == v) + (q.z == v) + (q.w == v);
+            }
             for (uint32_t i = STEPS; i < n; i++) c += path[i] == v;
             return c;
         };
         auto push = [&](uint32_t v) {
-            if (n < (uint32_t)STEPS) cache[n][tid] = v;
+            if (n < (uint32_t)STEPS) mine[n] = v;
             path[n] = v;
             atomicAdd(&a.freq[v], 1u);
             n++;
         };
 
         push(cur);
-        Corr c{1.0, 0.0, 0.0, 1.0, 0.0, 0.0, 1.0, 1.0};  // walk.hpp:853-855
+        uint32_t cur_visits = 1;
+        Corr c{0.0, 0.0, 0.0, 0.0};  // walk.hpp:853-855
         uint32_t attempt = 0;
+        uint64_t row = a.offsets[cur], end = a.offsets[cur + 1];
         for (;;) {
-            const uint64_t row = a.offsets[cur];
-            const uint32_t deg = (uint32_t)(a.offsets[cur + 1] - row);
+            const uint32_t deg = (uint32_t)(end - row);
             if (deg == 0) break;  // walk.hpp:887-892
             const uint4 x = philox4x32_10(make_uint4(attempt, w, a.round, kWalkTag), a.seed_lo, a.seed_hi);
             attempt++;
@@ -128,20 +162,28 @@ __global__ void __launch_bounds__(THREADS) walk_kernel(WalkArgs a) {
             n_trace += trace;
             const uint32_t dst = ent.x;
             if (n == a.stride) { n_over++; break; }
+            if (!trace) {   // the next row, while this footprint is counted
+                row = a.offsets[dst];
+                end = a.offsets[dst + 1];
+            }
             uint32_t fi = visit_count(dst);
             double t = a.etable[(uint64_t)n * (n + 1) / 2 + fi - 1];
+            double4 st = a.steps[n + 1];
+            corr_iterate(c, t, n, st);
             push(dst);
-            corr_iterate(c, t);
-            if (corr_stop(c, n - 1, a.min_len)) break;
+            if (corr_stop(c, n - 1, a.min_len, st)) break;
             if (trace) {  // walk.hpp:986-1017: step back to the current vertex
                 if (n == a.stride) { n_over++; break; }
-                fi = visit_count(cur);
-                t = a.etable[(uint64_t)n * (n + 1) / 2 + fi - 1];
+                cur_visits += dst == cur;
+                t = a.etable[(uint64_t)n * (n + 1) / 2 + cur_visits - 1];
+                cur_visits++;
+                st = a.steps[n + 1];
+                corr_iterate(c, t, n, st);
                 push(cur);
-                corr_iterate(c, t);
-                if (corr_stop(c, n - 1, a.min_len)) break;
+                if (corr_stop(c, n - 1, a.min_len, st)) break;
             } else {
                 cur = dst;
+                cur_visits = fi + 1;
             }
         }
         a.lens[w] = n;
@@ -312,6 +354,7 @@ int run_round(dg_graph *g, const dg_walk_params *p, uint32_t round, uint32_t n_w
     a.offsets = g->offsets.p;
     a.entries = g->entries.p;
     a.etable = g->etable.p;
+    a.steps = g->step_table.p;
     a.verts = ps->verts.p;
     a.lens = ps->lens.p;
     a.freq = g->freq.p;

@@ -64,12 +64,29 @@ __device__ __forceinline__ void adj_load(const float *f32, const __nv_bfloat16 *
     constexpr int D = 32 * V;
     if (f32 || w < n_master) {
         const float *p = (f32 ? f32 : master) + (size_t)w * D + col;
+        if constexpr (V % 4 == 0) {
 #pragma unroll
-        for (int c = 0; c < V; c++) x[c] = p[c];
+            for (int c = 0; c < V; c += 4) {
+                const float4 q = *reinterpret_cast<const float4 *>(p + c);
+                x[c] = q.x; x[c + 1] = q.y; x[c + 2] = q.z; x[c + 3] = q.w;
+            }
+        } else if constexpr (V == 2) {
+            const float2 q = *reinterpret_cast<const float2 *>(p);
+            x[0] = q.x; x[1] = q.y;
+        } else {
+            x[0] = p[0];
+        }
     } else {
         const __nv_bfloat16 *p = bf + (size_t)w * D + col;
+        if constexpr (V % 2 == 0) {
 #pragma unroll
-        for (int c = 0; c < V; c++) x[c] = __bfloat162float(p[c]);
+            for (int c = 0; c < V; c += 2) {
+                const float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(p + c));
+                x[c] = q.x; x[c + 1] = q.y;
+            }
+        } else {
+            x[0] = __bfloat162float(p[0]);
+        }
     }
 }
 
@@ -93,20 +110,47 @@ __device__ __forceinline__ void fix_add(unsigned long long *p, float x, unsigned
     atomicAdd(p, (unsigned long long)__float2ll_rn(x * kFixScale));
 }
 
+// acc[0 .. 32 V) += a row held V consecutive columns to a lane.  The sums are 8 bytes
+// wide, so lanes adding their own columns would touch a 32-byte sector each, V times
+// over; the row goes through shared memory (tmp, this warp's 32 V floats) and lane l
+// adds columns l, l + 32, ..., four to a sector.
+template <int V>
+__device__ __forceinline__ void fix_add_row(unsigned long long *acc, const float (&x)[V], float *tmp, int lane,
+                                            unsigned int *flag) {
+    if constexpr (V == 1) {
+        fix_add(acc + lane, x[0], flag);
+    } else {
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < V; c++) tmp[lane * V + c] = x[c];
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < V; c++) fix_add(acc + 32 * c + lane, tmp[32 * c + lane], flag);
+    }
+}
+
 __device__ __forceinline__ float fix_value(unsigned long long q) { return (float)((double)(long long)q * kFixInv); }
 
 // NEG > 0: the negative count fixed at compile time (a.negative == NEG); the
 // 1 + NEG dot products of a pair are then reduced together (warp_sums_split,
 // bit-identical to adj_dot) and each lane group evaluates one sigmoid.
 // NEG == 0: any count up to kAdjMaxNeg, one target after the other.
+//
+// A pair's 1 + neg loss terms are evaluated in FP64 side by side, a lane (group)
+// each, and added in the sequential order: evaluated one after the other by every
+// lane they were most of the kernel (about 1,200 FP64 instructions a pair).  What
+// bounds it now is the latency of a pair (row, sums, sigmoid, accumulators) at the
+// minibatches the GPU holds; the next pair's input row is loaded a pair ahead.
+// 200,000 pairs in minibatches of 21 on 50,000 rows of 128 columns: 452 -> 184 us.
 template <int V, int NEG>
 __global__ void __launch_bounds__(kAdjThreads) sgns_adjoint_kernel(AdjArgs a) {
     constexpr int D = 32 * V;
     extern __shared__ __align__(16) float adj_smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, col = lane * V;
     const int neg = NEG > 0 ? NEG : a.negative;
-    float *uk = adj_smem + (size_t)wib * 2 * neg * D;   // [neg][D] negative rows
-    float *gk = uk + (size_t)neg * D;                    // [neg][D] their gradient sums
+    float *uk = adj_smem + (size_t)wib * (2 * neg + 1) * D;   // [neg][D] negative rows
+    float *gk = uk + (size_t)neg * D;                          // [neg][D] their gradient sums
+    float *tmp = gk + (size_t)neg * D;                         // [D] a row on its way to an accumulator
     uint64_t n_pairs = a.n_pairs, b_begin = a.b_begin, b_end = a.b_end;
     if (a.step) {
         const AdjStep st = *a.step;
@@ -118,6 +162,7 @@ __global__ void __launch_bounds__(kAdjThreads) sgns_adjoint_kernel(AdjArgs a) {
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32);
     for (uint64_t b = b_begin + (uint64_t)blockIdx.x * (blockDim.x / 32) + wib; b < b_end; b += warps) {
         const uint64_t p0 = b * a.batch, p1 = min(p0 + a.batch, n_pairs);
+        __syncwarp();
         for (int k = 0; k < neg; k++) {
             float x[V];
             adj_load<V>(a.out_f32, a.out_bf, a.out_master, a.n_master, a.negatives[b * neg + k], col, x);
@@ -133,20 +178,30 @@ __global__ void __launch_bounds__(kAdjThreads) sgns_adjoint_kernel(AdjArgs a) {
         // order over the run, then added to the accumulator once.
         uint32_t run_o = 0xFFFFFFFFu;
         float uo[V], duo[V];
+        uint32_t ids_i = 0, ids_o = 0;   // lane l: the ids of pair l of a run of 32
+        float vn[V];                     // the next pair's input row
         for (uint64_t p = p0; p < p1; p++) {
-            const uint32_t i = a.inputs[p], o = a.outputs[p];
-            if (o != run_o) {
-                if (run_o != 0xFFFFFFFFu) {
-#pragma unroll
-                    for (int c = 0; c < V; c++) fix_add(a.acc_out + (size_t)run_o * D + col + c, duo[c], a.flag);
+            const int at = (int)(p - p0) & 31;
+            if (at == 0) {
+                if (p + lane < p1) {
+                    ids_i = a.inputs[p + lane];
+                    ids_o = a.outputs[p + lane];
                 }
+                adj_load<V>(a.in_f32, a.in_bf, a.in_master, a.n_master, __shfl_sync(0xffffffffu, ids_i, 0), col, vn);
+            }
+            const uint32_t i = __shfl_sync(0xffffffffu, ids_i, at), o = __shfl_sync(0xffffffffu, ids_o, at);
+            if (o != run_o) {
+                if (run_o != 0xFFFFFFFFu) fix_add_row<V>(a.acc_out + (size_t)run_o * D, duo, tmp, lane, a.flag);
                 adj_load<V>(a.out_f32, a.out_bf, a.out_master, a.n_master, o, col, uo);
 #pragma unroll
                 for (int c = 0; c < V; c++) duo[c] = 0.f;
                 run_o = o;
             }
             float v[V], dv[V];
-            adj_load<V>(a.in_f32, a.in_bf, a.in_master, a.n_master, i, col, v);
+#pragma unroll
+            for (int c = 0; c < V; c++) v[c] = vn[c];
+            if (at < 31 && p + 1 < p1)
+                adj_load<V>(a.in_f32, a.in_bf, a.in_master, a.n_master, __shfl_sync(0xffffffffu, ids_i, at + 1), col, vn);
             if constexpr (NEG > 0) {
                 constexpr int M = pow2_at_least(NEG + 1);
                 constexpr int GROUP = 32 / M;
@@ -176,10 +231,10 @@ __global__ void __launch_bounds__(kAdjThreads) sgns_adjoint_kernel(AdjArgs a) {
                 float g[NEG + 1];
 #pragma unroll
                 for (int k = 0; k <= NEG; k++) g[k] = __shfl_sync(0xffffffffu, gm, k * GROUP);
-                if (a.batch_loss) {   // the loss in the sequential order (every lane holds every sum)
-                    loss += softplus(-(double)__shfl_sync(0xffffffffu, mine, 0));
+                if (a.batch_loss) {   // a term per lane group, added in the sequential order
+                    const double term = softplus(jm == 0 ? -(double)mine : (double)mine);
 #pragma unroll
-                    for (int k = 0; k < NEG; k++) loss += softplus((double)__shfl_sync(0xffffffffu, mine, (k + 1) * GROUP));
+                    for (int k = 0; k <= NEG; k++) loss += __shfl_sync(0xffffffffu, term, k * GROUP);
                 }
 #pragma unroll
                 for (int c = 0; c < V; c++) {
@@ -194,13 +249,12 @@ __global__ void __launch_bounds__(kAdjThreads) sgns_adjoint_kernel(AdjArgs a) {
                         gk[k * D + col + c] = fmaf(g[k + 1], v[c], gk[k * D + col + c]);
                     }
                 }
-#pragma unroll
-                for (int c = 0; c < V; c++) fix_add(a.acc_in + (size_t)i * D + col + c, dv[c], a.flag);
+                fix_add_row<V>(a.acc_in + (size_t)i * D, dv, tmp, lane, a.flag);
                 continue;
             }
             const float s = adj_dot<V>(v, uo);
             const float g = -1.f / (1.f + expf(s));   // sigmoid(s) - 1
-            if (a.batch_loss) loss += softplus(-(double)s);
+            float mine = s;                            // lane k: the sum of target k (0: the positive)
 #pragma unroll
             for (int c = 0; c < V; c++) {
                 dv[c] = __fmul_rn(g, uo[c]);
@@ -212,24 +266,25 @@ __global__ void __launch_bounds__(kAdjThreads) sgns_adjoint_kernel(AdjArgs a) {
                 for (int c = 0; c < V; c++) u[c] = uk[k * D + col + c];
                 const float sk = adj_dot<V>(v, u);
                 const float gn = 1.f / (1.f + expf(-sk));   // sigmoid(s_k)
-                if (a.batch_loss) loss += softplus((double)sk);
+                if (lane == k + 1) mine = sk;
 #pragma unroll
                 for (int c = 0; c < V; c++) {
                     dv[c] = fmaf(gn, u[c], dv[c]);
                     gk[k * D + col + c] = fmaf(gn, v[c], gk[k * D + col + c]);
                 }
             }
-#pragma unroll
-            for (int c = 0; c < V; c++) fix_add(a.acc_in + (size_t)i * D + col + c, dv[c], a.flag);
+            if (a.batch_loss) {
+                const double term = softplus(lane == 0 ? -(double)mine : (double)mine);
+                for (int k = 0; k <= neg; k++) loss += __shfl_sync(0xffffffffu, term, k);
+            }
+            fix_add_row<V>(a.acc_in + (size_t)i * D, dv, tmp, lane, a.flag);
         }
-        if (run_o != 0xFFFFFFFFu) {
-#pragma unroll
-            for (int c = 0; c < V; c++) fix_add(a.acc_out + (size_t)run_o * D + col + c, duo[c], a.flag);
-        }
+        if (run_o != 0xFFFFFFFFu) fix_add_row<V>(a.acc_out + (size_t)run_o * D, duo, tmp, lane, a.flag);
+        __syncwarp();   // other lanes' columns of gk
         for (int k = 0; k < neg; k++) {
             const uint32_t w = a.negatives[b * neg + k];
 #pragma unroll
-            for (int c = 0; c < V; c++) fix_add(a.acc_out + (size_t)w * D + col + c, gk[k * D + col + c], a.flag);
+            for (int c = 0; c < V; c++) fix_add(a.acc_out + (size_t)w * D + 32 * c + lane, gk[k * D + 32 * c + lane], a.flag);
         }
         if (lane == 0 && a.batch_loss) a.batch_loss[b] = loss;
     }
@@ -326,7 +381,7 @@ struct AdjLaunch {
 
 template <int V>
 int adjoint_config(dg_sgns *s, int negative, uint64_t n_batches, AdjLaunch &l) {
-    const size_t per_warp = (size_t)2 * negative * 32 * V * sizeof(float);
+    const size_t per_warp = (size_t)(2 * negative + 1) * 32 * V * sizeof(float);
     int warps = kAdjThreads / 32;
     while (warps > 1 && per_warp * warps > 96 * 1024) warps /= 2;
     l.smem = per_warp * warps;

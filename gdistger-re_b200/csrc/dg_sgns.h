@@ -209,6 +209,7 @@ struct dg_sgns {
     uint64_t adj_exec_k = 0;
     dg::DevArray<int32_t> hs_off, hs_point;   // hierarchical softmax: Huffman paths (dgs::huffman_codes)
     dg::DevArray<int8_t> hs_code;
+    dg::DevArray<float> hs_hot;               // CBOW: rows of the nodes near the root during a launch (dg_sgns_cbow.cu)
     dg::DevArray<uint32_t> queue;
     dg::DevArray<unsigned long long> stats;
     dg::DevArray<uint64_t> host_off;     // dg_sgns_train_host: device copies of the caller's walks,

@@ -43,6 +43,28 @@ constexpr int kCbowPairNeg = 8;           // the largest negative count of this 
 constexpr int cbow_pair_walks(int vec) { return vec <= 4 ? 2 : 1; }    // walks that a warp trains in turn
 constexpr int cbow_pair_blocks(int vec) { return vec <= 4 ? 2 : 1; }   // blocks per SM
 
+// Hierarchical softmax: the table's kHotNodes last rows, spread.
+constexpr uint32_t kHotNodes = 64;
+constexpr uint32_t kHotPiece = 256;   // floats from one piece of a row to the next: the L2's slices change
+constexpr uint32_t kHotFloats = kHotNodes * 8 * kHotPiece;
+
+// Floats from the buffer's start to lane l's columns of hot row r: four lanes to a piece.
+template <int VEC>
+__device__ __forceinline__ uint32_t hot_offset(uint32_t r, uint32_t l) {
+    static_assert(4 * VEC <= (int)kHotPiece, "a piece holds four lanes' columns");
+    return (r * 8 + (l >> 2)) * kHotPiece + (l & 3) * VEC;
+}
+
+// Output rows [from, from + gridDim.x) into the buffer (in) or back, a warp per row.
+template <int VEC>
+__global__ void cbow_hot_rows(float *syn1, float *hot, int32_t from, bool in) {
+    float *row = syn1 + (size_t)(from + blockIdx.x) * (32 * VEC) + threadIdx.x * VEC;
+    float *at = hot + hot_offset<VEC>(blockIdx.x, threadIdx.x);
+    RowVec<VEC> r;
+    load_row<VEC>(in ? row : at, r);
+    store_row<VEC>(in ? at : row, r);
+}
+
 // A walk under way: its length, its next centre, and for token / centre `lane` the
 // word, the positions that hold the same word, the window as a mask of positions
 // and the targets' flags (bit j: target j trains, 0 being the centre's word; bit
@@ -65,9 +87,20 @@ struct CbowWalk {
 // starts, after the reductions of the centre before.
 //
 // NS: the negatives at compile time (5), or up to 8 read from a.negative.
+//
+// HS: hierarchical softmax over the centre's Huffman path before its targets
+// (word2vec.cu:436-455; hs_path, dg_sgns_dev.cuh).  Every path runs through the
+// nodes near the root, and what bounds it is that the L2 serves one row's read and
+// reduction per 8.3 ns as long as both rows of a kilobyte are one slice's work: the
+// root and its two neighbours cost 1.1M tokens 9 ms of 10.3.  So for the launch the
+// kHotNodes most visited nodes' rows (the last inner nodes made, so the highest ids)
+// move to a buffer whose rows lie in eight pieces a kilobyte apart (hot_offset),
+// each another slice's, and a path's nodes are read four at a time.
+// A round of the 50,000-vertex graph, size 128, window 5, with its read-back:
+// 11.4 -> 7.2 ms.
 template <int VEC, int NS, bool HS>
 __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
-    sgns_cbow_pair_kernel(SgnsArgs a, WalkSet ws, uint32_t walks) {
+    sgns_cbow_pair_kernel(SgnsArgs a, WalkSet ws, uint32_t walks, float *hot, int32_t hot_from) {
     constexpr int D = 32 * VEC, M = pow2_at_least(NS + 1), GROUP = 32 / M;
     constexpr int BATCH = VEC <= 4 ? 8 : 4;   // context rows in flight together
     constexpr uint32_t kAll = 0xffffffffu;
@@ -80,6 +113,11 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
     // the next power of two) read lane 0's columns, hold x = 0 and write nothing.
     const bool own = lane * VEC < (uint32_t)a.used;
     float *const syn0 = a.syn0 + (own ? lane * VEC : 0), *const syn1 = a.syn1 + (own ? lane * VEC : 0);
+    // This lane's columns of output row `id`.
+    auto out_row = [&](int32_t id) {
+        if (HS && id >= hot_from) return hot + hot_offset<VEC>((uint32_t)(id - hot_from), own ? lane : 0);
+        return syn1 + (size_t)id * D;
+    };
     unsigned long long n_words = 0, n_trained = 0, n_pairs = 0;
     CbowWalk A, B;
     A.sen = sen_all[warp][0];
@@ -142,7 +180,7 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
         for (int j = 0; j < NS; j++) q.t[j + 1] = j < neg ? A.negs[p * NS + j] : q.t[0];
 #pragma unroll
         for (int j = 0; j <= NS; j++)
-            if (j <= neg) load_row<VEC>(syn1 + (size_t)q.t[j] * D, q.row[j]);
+            if (j <= neg) load_row<VEC>(out_row(q.t[j]), q.row[j]);
     };
     // The target rows of centre p of walk W on their way to L2, a lane per row.
     auto prefetch_targets = [&](const CbowWalk &W, uint32_t p) {
@@ -166,7 +204,7 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
                 const float g = __shfl_sync(kAll, gm, j * GROUP);
                 if (!((fl >> j) & 1u)) continue;
                 row_fma(e, g, q.row[j]);
-                if (own) add_row<VEC>(syn1 + (size_t)q.t[j] * D, row_mul(g, x));
+                if (own) add_row<VEC>(out_row(q.t[j]), row_mul(g, x));
             }
         } else {   // a target repeats: one after the other, each seeing the updates before it
 #pragma unroll
@@ -176,7 +214,7 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
                 row_fma(e, g, q.row[j]);
                 const RowVec<VEC> upd = row_mul(g, x);
                 row_add(q.row[j], upd);
-                if (own) add_row<VEC>(syn1 + (size_t)q.t[j] * D, upd);
+                if (own) add_row<VEC>(out_row(q.t[j]), upd);
 #pragma unroll
                 for (int k = j + 1; k <= NS; k++)
                     if (q.t[k] == q.t[j]) q.row[k] = q.row[j];
@@ -191,6 +229,46 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
         for (int i = 0; i < VEC; i++) {
             const float q = x.v[i] * r;
             x.v[i] = own ? fmaf(fmaf(-q, cw, x.v[i]), r, q) : 0.f;
+        }
+    };
+
+    // Centre p's path against x: the nodes are distinct, so four are read, summed and
+    // updated together.
+    auto train_path = [&](uint32_t p, const RowVec<VEC> &x, RowVec<VEC> &e) {
+        constexpr int H = 4;
+        const int32_t word = A.sen[p], k1 = a.hs_off[word + 1];
+        for (int32_t k = a.hs_off[word]; k < k1; k += H) {
+            int32_t point = -1;
+            float label = 0.f;
+            if ((int)lane < H && k + (int32_t)lane < k1) {
+                point = a.hs_point[k + lane];
+                label = (float)(1 - a.hs_code[k + lane]);
+            }
+            int32_t node[H];
+            RowVec<VEC> row[H];
+            float f[H];
+#pragma unroll
+            for (int j = 0; j < H; j++) {
+                node[j] = __shfl_sync(kAll, point, j);
+                if (node[j] >= 0) load_row<VEC>(out_row(node[j]), row[j]);
+                else zero_row(row[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < H; j++) f[j] = row_dot(x, row[j]);
+            const float mine = warp_sums_split<H>(f, lane);
+            const float lab = __shfl_sync(kAll, label, lane / (32 / H));
+            const bool skip = mine <= -kMaxExp || mine >= kMaxExp;
+            float gm = 0.f;
+            if (!skip)
+                gm = (lab - __ldg(a.exp_table + (int)((mine + kMaxExp) * (kExpTableSize / kMaxExp / 2)))) * a.alpha;
+            const uint32_t skipped = __ballot_sync(kAll, skip);
+#pragma unroll
+            for (int j = 0; j < H; j++) {
+                const float g = __shfl_sync(kAll, gm, j * (32 / H));
+                if (node[j] < 0 || ((skipped >> (j * (32 / H))) & 1u)) continue;
+                row_fma(e, g, row[j]);
+                if (own) add_row<VEC>(out_row(node[j]), row_mul(g, x));
+            }
         }
     };
 
@@ -233,7 +311,7 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
             mean(x, wp);
             zero_row(e);
             if (HS) {
-                hs_path<VEC>(a, A.sen[p], x, e, lane);
+                train_path(p, x, e);
                 load_targets(p, q);
             }
             train_targets(p, x, e, q);
@@ -244,7 +322,7 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
                 mean(y, wq);
                 zero_row(x);   // from here the second centre's e
                 if (HS) {
-                    hs_path<VEC>(a, A.sen[p + 1], y, x, lane);
+                    train_path(p + 1, y, x);
                     load_targets(p + 1, q);
                 }
                 train_targets(p + 1, y, x, q);
@@ -295,8 +373,20 @@ static int cbow_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
     int blocks = std::min(std::max(per_sm, 1), cbow_pair_blocks(V)) * dg::sm_count(s->device);
     const uint32_t walks = want > 0 && want <= (uint32_t)(blocks * warps) ? 1u : (uint32_t)cbow_pair_walks(V);
     if (want > 0) blocks = std::min(blocks, std::max(1, (int)(want / (walks * (uint32_t)warps))));
-    kern<<<blocks, 32 * warps, 0, s->stream>>>(a, ws, walks);
+    // The last rows of the table: inner nodes are rows 0 .. vocabulary - 2, the root the last of them.
+    const uint32_t n_hot = HS ? std::min(kHotNodes, s->vocab_size) : 0;
+    const int32_t hot_from = HS ? (int32_t)(s->vocab_size - n_hot) : 0;
+    if (HS) {
+        if (s->hs_hot.n == 0) DG_CUDA(s->hs_hot.alloc(kHotFloats));
+        cbow_hot_rows<V><<<n_hot, 32, 0, s->stream>>>(s->syn1.p, s->hs_hot.p, hot_from, true);
+        dg::note_launch();
+    }
+    kern<<<blocks, 32 * warps, 0, s->stream>>>(a, ws, walks, s->hs_hot.p, hot_from);
     dg::note_launch();
+    if (HS) {
+        cbow_hot_rows<V><<<n_hot, 32, 0, s->stream>>>(s->syn1.p, s->hs_hot.p, hot_from, false);
+        dg::note_launch();
+    }
     DG_CUDA(cudaGetLastError());
     return DG_OK;
 }

@@ -14,7 +14,7 @@
 //
 // A Hogwild run's rows depend on how many pairs are under way unseen and on how
 // many walks are trained at once (dg_sgns_cbow.cu), so half as many warps as
-// sgns_negshare_kernel's hold two walks each and train a centre of either in turn.
+// sgns_negshare_kernel's hold two walks each and train two pairs of either in turn.
 //
 // A round of the 50,000-vertex graph at size 200, window 5, negative 5, with its
 // read-back: 20.5 -> 12.6 ms.  The rows end 1.3 to 2 times as far from the one-pair
@@ -34,13 +34,37 @@ constexpr int kSharePairNeg = 8;           // the largest negative count of this
 // Blocks per SM: two walks a warp, 32 walks up to 128 columns, 16 at 256.
 constexpr int share_pair_blocks(int vec) { return vec <= 4 ? 2 : 1; }
 
-// A walk under way: its length and next centre, its words and negatives (shared),
-// and whether a negative occurs twice.
+// A walk under way: its length, centre and the centre's next pair, its words and
+// negatives (shared), whether a negative occurs twice, and this lane's columns of
+// the centre's output row, as it was read and as it is between turns (shared).
 struct ShareWalk {
-    uint32_t n = 0, p = 0;
+    uint32_t n = 0, p = 0, k = 0;
     int32_t *sen = nullptr, *negs = nullptr;
+    float *pos0 = nullptr, *pos = nullptr;
     bool repeat = false;
 };
+
+template <int VEC>
+__device__ __forceinline__ void share_put(float *p, const RowVec<VEC> &r) {
+#pragma unroll
+    for (int i = 0; i < VEC; i += VEC >= 4 ? 4 : 2) {
+        if constexpr (VEC >= 4) *reinterpret_cast<float4 *>(p + i) = make_float4(r.v[i], r.v[i + 1], r.v[i + 2], r.v[i + 3]);
+        else *reinterpret_cast<float2 *>(p + i) = make_float2(r.v[i], r.v[i + 1]);
+    }
+}
+template <int VEC>
+__device__ __forceinline__ void share_get(const float *p, RowVec<VEC> &r) {
+#pragma unroll
+    for (int i = 0; i < VEC; i += VEC >= 4 ? 4 : 2) {
+        if constexpr (VEC >= 4) {
+            const float4 q = *reinterpret_cast<const float4 *>(p + i);
+            r.v[i] = q.x; r.v[i + 1] = q.y; r.v[i + 2] = q.z; r.v[i + 3] = q.w;
+        } else {
+            const float2 q = *reinterpret_cast<const float2 *>(p + i);
+            r.v[i] = q.x; r.v[i + 1] = q.y;
+        }
+    }
+}
 
 // Lane l owns columns [l * VEC, l * VEC + VEC) of every row.  NS: the negatives at
 // compile time (5), or up to 8 read from a.negative.
@@ -59,14 +83,20 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
     float *const syn0 = a.syn0 + (own ? lane * VEC : 0), *const syn1 = a.syn1 + (own ? lane * VEC : 0);
     unsigned long long n_words = 0, n_trained = 0, n_pairs = 0;
     ShareWalk A, B;
+    extern __shared__ __align__(16) float share_smem[];   // per walk the centre's row, twice
+    float *const rows = share_smem + (size_t)warp * 4 * D + lane * VEC;
     A.sen = sen_all[warp][0];
     A.negs = negs_all[warp][0];
+    A.pos0 = rows;
+    A.pos = rows + D;
     B.sen = sen_all[warp][1];
     B.negs = negs_all[warp][1];
+    B.pos0 = rows + 2 * D;
+    B.pos = rows + 3 * D;
     bool more = true;
 
     auto fetch = [&]() {   // the next walk of at least two tokens into A; A.n = 0 when there is none left
-        A.n = A.p = 0;
+        A.n = A.p = A.k = 0;
         while (more) {
             uint32_t walk = 0;
             if (lane == 0) walk = atomicAdd(a.queue, 1u);
@@ -102,9 +132,13 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
         if (A.n) {
             const uint32_t p = A.p, n = A.n;
             const int32_t word = A.sen[p];
-            RowVec<VEC> pos, pos0;
-            load_row<VEC>(syn1 + (size_t)word * D, pos);
-            pos0 = pos;
+            RowVec<VEC> pos;
+            if (A.k == 0) {
+                load_row<VEC>(syn1 + (size_t)word * D, pos);
+                share_put(A.pos0, pos);
+            } else {
+                share_get(A.pos, pos);
+            }
             int32_t t[NS];
             uint32_t live = 0;   // bit j: negative j trains (it is not the centre's word)
 #pragma unroll
@@ -114,7 +148,6 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
             }
             const uint32_t lo = p > w ? p - w : 0u, hi = min(n, p + w + 1);   // positions; p itself is no context
             const uint32_t m = hi - lo - 1;
-            n_pairs += m;
             auto at = [&](uint32_t k) { return A.sen[lo + k + (lo + k >= p ? 1u : 0u)]; };
             // The gradients of the pair (l, centre): lane group j holds negative j's, group neg's the
             // positive's; all sums are of the rows as they are.
@@ -128,8 +161,10 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
                 if (jm == (uint32_t)NS || ((live >> jm) & 1u)) g = sg_grad(mine, jm == (uint32_t)NS, a.exp_table, a.alpha);
                 return g;
             };
+            const uint32_t k = A.k;   // this turn's pairs: k and, where there is one, k + 1
+            n_pairs += min(2u, m - k);
             if (!A.repeat) {
-                for (uint32_t k = 0; k < m; k += 2) {
+                {
                     const bool two = k + 1 < m;
                     const int32_t w1 = at(k), w2 = two ? at(k + 1) : w1;
                     RowVec<VEC> l1, l2, e, row[NS];
@@ -175,8 +210,8 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
                     }
                 }
             } else {   // a negative occurs twice: one target after the other
-                for (uint32_t k = 0; k < m; k++) {
-                    const int32_t w1 = at(k);
+                for (uint32_t c = k; c < min(k + 2, m); c++) {
+                    const int32_t w1 = at(c);
                     RowVec<VEC> l1, e;
                     load_context(w1, l1);
                     zero_row(e);
@@ -195,10 +230,18 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
                     if (own) add_row<VEC>(syn0 + (size_t)w1 * D, e);
                 }
             }
+            A.k = k + 2;
+            if (A.k < m) {
+                share_put(A.pos, pos);
+            } else {   // the centre is done
+                RowVec<VEC> was;
+                share_get(A.pos0, was);
 #pragma unroll
-            for (int i = 0; i < VEC; i++) pos.v[i] -= pos0.v[i];
-            if (own) add_row<VEC>(syn1 + (size_t)word * D, pos);
-            A.p = p + 1;
+                for (int i = 0; i < VEC; i++) pos.v[i] -= was.v[i];
+                if (own) add_row<VEC>(syn1 + (size_t)word * D, pos);
+                A.p = p + 1;
+                A.k = 0;
+            }
         }
         if (walks > 1) {
             const ShareWalk x = A;
@@ -224,11 +267,13 @@ static int negshare_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws
     const uint32_t want = s->p.workers;   // the caller's bound on walks under way: a warp each, or two if need be
     const int warps = want > 0 && want < (uint32_t)kShareWarps ? (int)want : kShareWarps;
     int per_sm = 0;
-    DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, 0));
+    const size_t smem = (size_t)warps * 4 * 32 * V * sizeof(float);
+    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem));
     int blocks = std::min(std::max(per_sm, 1), share_pair_blocks(V)) * dg::sm_count(s->device);
     const uint32_t walks = want > 0 && want <= (uint32_t)(blocks * warps) ? 1u : 2u;
     if (want > 0) blocks = std::min(blocks, std::max(1, (int)(want / (walks * (uint32_t)warps))));
-    kern<<<blocks, 32 * warps, 0, s->stream>>>(a, ws, walks);
+    kern<<<blocks, 32 * warps, smem, s->stream>>>(a, ws, walks);
     dg::note_launch();
     DG_CUDA(cudaGetLastError());
     return DG_OK;

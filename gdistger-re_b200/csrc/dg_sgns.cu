@@ -456,7 +456,12 @@ __global__ void __launch_bounds__(THREADS, FIT > 0 ? FIT : 1) sgns_plain_kernel(
 //    finished centre) updated it misses that update: staleness of at most S
 //    pairs, of the kind other warps' concurrent updates cause in any Hogwild run.
 // Draws, pairs, sums, gradients and the update order of each pair are
-// sgns_plain_kernel's.  The launcher uses it only without `deterministic`, for
+// sgns_plain_kernel's.  The default shape's twelve blocks per SM leave 80 registers,
+// and what spills is paid at every pair, so BF16 rows keep the run's counts in
+// shared memory, a walk at a time (100,000 walks of the YouTube-shaped graph: 13.76
+// -> 13.68 ms at five negatives, 28.3 -> 26.7 at three, 39.1 -> 37.1 at eight).  FP32
+// rows are faster with theirs in registers: ptxas finds a worse allocation without
+// (15.8 -> 20.1 ms; time both after any change here).  The launcher uses it only without `deterministic`, for
 // sentences of at most kPipeSentence tokens, window <= kPipeMaxWindow and
 // negative <= kFastNeg.
 constexpr uint32_t kPipeSentence = 64;
@@ -563,6 +568,8 @@ __global__ void __launch_bounds__(THREADS, FIT > 0 ? FIT : 1) sgns_plain_pipe_ke
     constexpr int GROUP = 32 / M;
     __shared__ PipeWarp<VEC, NS, S> sm_all[THREADS / 32];
     PipeWarp<VEC, NS, S> &sm = sm_all[threadIdx.x >> 5];
+    __shared__ unsigned long long counts_all[BF ? THREADS / 32 : 1][3];   // BF16 rows: words, trained, pairs of a warp
+    unsigned long long *const counts = counts_all[BF ? threadIdx.x >> 5 : 0];
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t w = (uint32_t)a.window;
     const float alpha = a.alpha;
@@ -570,7 +577,11 @@ __global__ void __launch_bounds__(THREADS, FIT > 0 ? FIT : 1) sgns_plain_pipe_ke
     const BfRows<VEC> in{a.in_bf, a.in_master, a.n_master, D};
     const BfRows<VEC> out{a.out_bf, a.out_master, a.n_master, D};
     const uint32_t key = a.seed_lo ^ bf_mix(a.pass * 0x9E3779B9u + 0x2F6B3A91u);
-    unsigned long long n_words = 0, n_trained = 0, n_pairs = 0;
+    unsigned long long n_words = 0, n_trained = 0, n_pairs = 0;   // BF16 rows: in counts
+    if constexpr (BF) {
+        if (lane < 3) counts[lane] = 0;
+        __syncwarp();
+    }
     int32_t hw[S];   // context words of this warp's last S pairs, newest first
 #pragma unroll
     for (int k = 0; k < S; k++) hw[k] = -1;
@@ -599,14 +610,25 @@ __global__ void __launch_bounds__(THREADS, FIT > 0 ? FIT : 1) sgns_plain_pipe_ke
         const uint32_t wid = ws.ids ? ws.ids[walk] : walk + ws.id_base;
         uint32_t words;
         const uint32_t n = warp_sentence<kPipeSentence>(ws, walk, a, sm.sen, words);
-        n_words += words;
-        n_trained += n;
+        if constexpr (!BF) {
+            n_words += words;
+            n_trained += n;
+        } else if (lane == 0) {
+            counts[0] += words;
+            counts[1] += n;
+        }
         if (n < 2) continue;   // a one-token sentence has no pairs
+        uint32_t pairs = 0;
         for (uint32_t q = lane; q < n; q += 32) {
             const uint32_t b = philox(q, wid, a.pass, kWinTag, a.seed_lo, a.seed_hi).x % w;
             uint32_t lo, hi;
             slot_range(q, n, w, b, lo, hi);
             sm.lohi[q] = (uint16_t)(lo | (hi << 8));
+            if (BF) pairs += hi - lo - 1;   // slot w lies inside the range
+        }
+        if constexpr (BF) {
+            pairs = __reduce_add_sync(0xffffffffu, pairs);
+            if (lane == 0) counts[2] += pairs;
         }
         __syncwarp();
         // With n >= 2 every centre has a pair, and slot w lies inside its range.
@@ -702,7 +724,7 @@ __global__ void __launch_bounds__(THREADS, FIT > 0 ? FIT : 1) sgns_plain_pipe_ke
             for (int j = 0; j < NS; j++) t[j] = j < neg ? tq[j] : -1;
 #pragma unroll
             for (int i = 0; i < VEC; i++) e.v[i] = 0.f;
-            n_pairs++;
+            if constexpr (!BF) n_pairs++;
             const uint32_t flags = sm.fl[p % S][ks];
             const bool repeat = (flags & 0x8000u) != 0;
             // Writes negative j's row: an atomic delta (FP32 rows, masters) or the
@@ -826,9 +848,9 @@ __global__ void __launch_bounds__(THREADS, FIT > 0 ? FIT : 1) sgns_plain_pipe_ke
         }
     }
     if (lane == 0) {
-        atomicAdd(&a.stats[0], n_words);
-        atomicAdd(&a.stats[1], n_trained);
-        atomicAdd(&a.stats[2], n_pairs);
+        atomicAdd(&a.stats[0], BF ? counts[0] : n_words);
+        atomicAdd(&a.stats[1], BF ? counts[1] : n_trained);
+        atomicAdd(&a.stats[2], BF ? counts[2] : n_pairs);
     }
 }
 

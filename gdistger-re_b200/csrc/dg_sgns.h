@@ -81,13 +81,13 @@ struct SgnsArgs {
     uint64_t train_words;
     uint32_t vocab_size;
     int window, negative, d;
-    int used;                           // columns of a row that are not padding (<= d)
     float alpha;
     uint32_t pass, seed_lo, seed_hi;
     int deterministic;
     int hs;                             // hierarchical softmax: Huffman paths below
     const int32_t *hs_off, *hs_point;   // [vocab + 1] code-length prefix; inner node per bit
     const int8_t *hs_code;              // bit per path entry
+    int used;                           // columns of a row that are not padding (<= d)
 };
 
 // Warp sums of M per-lane partials v[0..M) (M a power of two <= 32) for the cost

@@ -17,7 +17,7 @@
 // sgns_negshare_kernel's hold two walks each and train two pairs of either in turn.
 //
 // A round of the 50,000-vertex graph at size 200, window 5, negative 5, with its
-// read-back: 20.5 -> 12.6 ms.  The rows end 1.3 to 2 times as far from the one-pair
+// read-back: 20.5 -> 11.6 ms.  The rows end 1.1 to 1.5 times as far from the one-pair
 // kernel's as two equal runs of that kernel from each other.
 #include "dg_sgns.h"
 #include "dg_sgns_dev.cuh"

@@ -21,33 +21,35 @@
 
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <memory>
 
 namespace {
 
-__global__ void cn_keys(const uint32_t *src, const uint32_t *dst, uint64_t n, int undirected, uint64_t *dir,
+// Keys of two ids in 2 * bits bits: the sorts pass over no others.
+__global__ void cn_keys(const uint32_t *src, const uint32_t *dst, uint64_t n, int undirected, int bits, uint64_t *dir,
                         uint64_t *pair, uint64_t *idx) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t s = src[i], d = dst[i];
         if (undirected) {
-            dir[2 * i] = (s << 32) | d;
-            dir[2 * i + 1] = (d << 32) | s;
+            dir[2 * i] = (s << bits) | d;
+            dir[2 * i + 1] = (d << bits) | s;
         } else {
-            dir[i] = (s << 32) | d;
+            dir[i] = (s << bits) | d;
         }
-        pair[i] = s < d ? (s << 32) | d : (d << 32) | s;
+        pair[i] = s < d ? (s << bits) | d : (d << bits) | s;
         idx[i] = i;
     }
 }
 
-__global__ void cn_rows(const uint64_t *dir, uint64_t m, uint32_t v_num, uint64_t *offsets, uint32_t *nbr) {
+__global__ void cn_rows(const uint64_t *dir, uint64_t m, uint32_t v_num, int bits, uint64_t *offsets, uint32_t *nbr) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t src = (uint32_t)(dir[i] >> 32);
-        const int64_t prev = i == 0 ? -1 : (int64_t)(dir[i - 1] >> 32);
+        const uint32_t src = (uint32_t)(dir[i] >> bits);
+        const int64_t prev = i == 0 ? -1 : (int64_t)(dir[i - 1] >> bits);
         for (int64_t v = prev + 1; v <= (int64_t)src; v++) offsets[v] = i;
         if (i == m - 1)
             for (uint64_t v = (uint64_t)src + 1; v <= v_num; v++) offsets[v] = m;
-        nbr[i] = (uint32_t)dir[i];
+        nbr[i] = (uint32_t)(dir[i] & (((uint64_t)1 << bits) - 1));
     }
 }
 
@@ -118,14 +120,11 @@ __global__ void cn_scatter(const uint64_t *pair_sorted, const uint64_t *idx_sort
     }
 }
 
-template <typename F>
-int cub_call(F f) {
-    size_t bytes = 0;
-    DG_CUDA(f(nullptr, bytes));
-    dg::DevArray<uint8_t> tmp;
-    DG_CUDA(tmp.alloc(bytes ? bytes : 1));
-    DG_CUDA(f(tmp.p, bytes));
-    return DG_OK;
+// Bits that hold every id below v_num.
+int bits_of(uint32_t v_num) {
+    int b = 1;
+    while (b < 32 && ((uint64_t)1 << b) < v_num) b++;
+    return b;
 }
 
 }  // namespace
@@ -134,9 +133,12 @@ extern "C" int dg_common_neighbours(const uint32_t *src, const uint32_t *dst, ui
                                     int undirected, int device, int32_t *cn) {
     DG_CHECK(n_edges == 0 || (src && dst && cn), DG_ERR_ARG, "dg_common_neighbours: NULL argument");
     DG_CHECK(v_num > 0, DG_ERR_ARG, "dg_common_neighbours: v_num must be positive");
-    for (uint64_t i = 0; i < n_edges; i++)
-        DG_CHECK(src[i] < v_num && dst[i] < v_num, DG_ERR_ARG, "edge %llu (%u, %u) has a vertex id >= v_num = %u",
-                 (unsigned long long)i, src[i], dst[i], v_num);
+    uint32_t top = 0;   // the largest id: a loop the compiler vectorises
+    for (uint64_t i = 0; i < n_edges; i++) top = std::max(top, std::max(src[i], dst[i]));
+    if (top >= v_num)
+        for (uint64_t i = 0; i < n_edges; i++)
+            DG_CHECK(src[i] < v_num && dst[i] < v_num, DG_ERR_ARG, "edge %llu (%u, %u) has a vertex id >= v_num = %u",
+                     (unsigned long long)i, src[i], dst[i], v_num);
     if (n_edges == 0) return DG_OK;
     int n_dev = 0;
     DG_CUDA(cudaGetDeviceCount(&n_dev));
@@ -150,47 +152,53 @@ extern "C" int dg_common_neighbours(const uint32_t *src, const uint32_t *dst, ui
     } sg{s};
     const uint64_t n = n_edges, m = undirected ? 2 * n : n;
     const unsigned grid = (unsigned)dg::sm_count(device) * 8;
-    dg::DevArray<uint32_t> d_src, d_dst, nbr;
-    dg::DevArray<uint64_t> dir, dir2, pair, pair2, idx, idx2, offsets;
-    dg::DevArray<int32_t> cn_sorted, d_cn;
-    DG_CUDA(d_src.alloc(n));
-    DG_CUDA(d_dst.alloc(n));
-    DG_CUDA(cudaMemcpyAsync(d_src.p, src, n * 4, cudaMemcpyHostToDevice, s));
-    DG_CUDA(cudaMemcpyAsync(d_dst.p, dst, n * 4, cudaMemcpyHostToDevice, s));
-    DG_CUDA(dir.alloc(m));
-    DG_CUDA(dir2.alloc(m));
-    DG_CUDA(pair.alloc(n));
-    DG_CUDA(pair2.alloc(n));
-    DG_CUDA(idx.alloc(n));
-    DG_CUDA(idx2.alloc(n));
-    cn_keys<<<grid, 256, 0, s>>>(d_src.p, d_dst.p, n, undirected, dir.p, pair.p, idx.p);
+    // One allocation for everything (each costs hundreds of microseconds), cut into
+    // 256-byte aligned parts; the two sorts share the larger one's scratch.
+    const int key_bits = bits_of(v_num);
+    size_t cub_rows = 0, cub_pairs = 0;
+    DG_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, cub_rows, (uint64_t *)nullptr, (uint64_t *)nullptr, m, 0, 2 * key_bits, s));
+    DG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, cub_pairs, (uint64_t *)nullptr, (uint64_t *)nullptr,
+                                            (uint64_t *)nullptr, (uint64_t *)nullptr, n, 0, 2 * key_bits, s));
+    const size_t cub_bytes = std::max(cub_rows, cub_pairs);
+    size_t need = 0;
+    auto part = [&](size_t bytes) {
+        const size_t at = need;
+        need += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t o_src = part(n * 4), o_dst = part(n * 4), o_nbr = part(m * 4), o_off = part(((size_t)v_num + 1) * 8),
+                 o_dir = part(m * 8), o_dir2 = part(m * 8), o_pair = part(n * 8), o_pair2 = part(n * 8),
+                 o_idx = part(n * 8), o_idx2 = part(n * 8), o_sorted = part(n * 4), o_cn = part(n * 4),
+                 o_cub = part(cub_bytes ? cub_bytes : 1);
+    dg::DevArray<uint8_t> block;
+    DG_CUDA(block.alloc(need));
+    uint32_t *const d_src = reinterpret_cast<uint32_t *>(block.p + o_src), *const d_dst = reinterpret_cast<uint32_t *>(block.p + o_dst),
+             *const nbr = reinterpret_cast<uint32_t *>(block.p + o_nbr);
+    uint64_t *const offsets = reinterpret_cast<uint64_t *>(block.p + o_off), *const dir = reinterpret_cast<uint64_t *>(block.p + o_dir),
+             *const dir2 = reinterpret_cast<uint64_t *>(block.p + o_dir2), *const pair = reinterpret_cast<uint64_t *>(block.p + o_pair),
+             *const pair2 = reinterpret_cast<uint64_t *>(block.p + o_pair2), *const idx = reinterpret_cast<uint64_t *>(block.p + o_idx),
+             *const idx2 = reinterpret_cast<uint64_t *>(block.p + o_idx2);
+    int32_t *const cn_sorted = reinterpret_cast<int32_t *>(block.p + o_sorted), *const d_cn = reinterpret_cast<int32_t *>(block.p + o_cn);
+    DG_CUDA(cudaMemcpyAsync(d_src, src, n * 4, cudaMemcpyHostToDevice, s));
+    DG_CUDA(cudaMemcpyAsync(d_dst, dst, n * 4, cudaMemcpyHostToDevice, s));
+    cn_keys<<<grid, 256, 0, s>>>(d_src, d_dst, n, undirected, key_bits, dir, pair, idx);
     dg::note_launch();
     DG_CUDA(cudaGetLastError());
     // Row-sorted CSR (gcn.cpp:130-137 sorts every row by neighbour).
-    int rc = cub_call([&](void *t, size_t &b) {
-        return cub::DeviceRadixSort::SortKeys(t, b, dir.p, dir2.p, m, 0, 64, s);
-    });
-    if (rc) return rc;
-    DG_CUDA(offsets.alloc((size_t)v_num + 1));
-    DG_CUDA(nbr.alloc(m));
-    cn_rows<<<grid, 256, 0, s>>>(dir2.p, m, v_num, offsets.p, nbr.p);
+    size_t bytes = cub_bytes;
+    DG_CUDA(cub::DeviceRadixSort::SortKeys(block.p + o_cub, bytes, dir, dir2, m, 0, 2 * key_bits, s));
+    cn_rows<<<grid, 256, 0, s>>>(dir2, m, v_num, key_bits, offsets, nbr);
     dg::note_launch();
     DG_CUDA(cudaGetLastError());
-    dir.release();
-    dir2.release();
     // Pairs grouped by unordered key, input order kept inside a group (stable sort).
-    rc = cub_call([&](void *t, size_t &b) {
-        return cub::DeviceRadixSort::SortPairs(t, b, pair.p, pair2.p, idx.p, idx2.p, n, 0, 64, s);
-    });
-    if (rc) return rc;
-    DG_CUDA(cn_sorted.alloc(n));
-    DG_CUDA(d_cn.alloc(n));
-    cn_count<<<grid, 256, 0, s>>>(pair2.p, idx2.p, n, d_src.p, d_dst.p, offsets.p, nbr.p, cn_sorted.p);
+    bytes = cub_bytes;
+    DG_CUDA(cub::DeviceRadixSort::SortPairs(block.p + o_cub, bytes, pair, pair2, idx, idx2, n, 0, 2 * key_bits, s));
+    cn_count<<<grid, 256, 0, s>>>(pair2, idx2, n, d_src, d_dst, offsets, nbr, cn_sorted);
     dg::note_launch();
-    cn_scatter<<<grid, 256, 0, s>>>(pair2.p, idx2.p, n, cn_sorted.p, d_cn.p);
+    cn_scatter<<<grid, 256, 0, s>>>(pair2, idx2, n, cn_sorted, d_cn);
     dg::note_launch();
     DG_CUDA(cudaGetLastError());
-    DG_CUDA(cudaMemcpyAsync(cn, d_cn.p, n * 4, cudaMemcpyDeviceToHost, s));
+    DG_CUDA(cudaMemcpyAsync(cn, d_cn, n * 4, cudaMemcpyDeviceToHost, s));
     DG_CUDA(cudaStreamSynchronize(s));
     return DG_OK;
 }

@@ -120,19 +120,20 @@ __global__ void scan_tiles(const uint32_t *in, uint64_t n, const uint64_t *tile_
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == SCAN_THREADS - 1) out[n] = ex;
 }
 
-int exclusive_scan_u32_to_u64(const uint32_t *in, uint64_t *out, uint64_t n, cudaStream_t s) {
+int exclusive_scan_u32_to_u64(const uint32_t *in, uint64_t *out, uint64_t n, cudaStream_t s, DevArray<uint64_t> *kept) {
     if (n == 0) {
         DG_CUDA(cudaMemsetAsync(out, 0, sizeof(uint64_t), s));
         return DG_OK;
     }
     uint64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-    DevArray<uint64_t> sums;
-    DG_CUDA(sums.alloc(tiles));
+    DevArray<uint64_t> own;
+    DevArray<uint64_t> &sums = kept ? *kept : own;
+    if (sums.n < tiles) DG_CUDA(sums.alloc(tiles));
     scan_tile_sums<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(in, n, sums.p); dg::note_launch();
     scan_tile_offsets<<<1, SCAN_THREADS, 0, s>>>(sums.p, tiles); dg::note_launch();
     scan_tiles<<<(unsigned)tiles, SCAN_THREADS, 0, s>>>(in, n, sums.p, out); dg::note_launch();
     DG_CUDA(cudaGetLastError());
-    DG_CUDA(cudaStreamSynchronize(s));
+    if (!kept) DG_CUDA(cudaStreamSynchronize(s));
     return DG_OK;
 }
 

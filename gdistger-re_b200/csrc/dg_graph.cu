@@ -231,6 +231,9 @@ dg_graph::~dg_graph() {
         in_deg.release();
         freq.release();
         etable.release(); step_table.release();
+        if (round_host) cudaFreeHost(round_host);
+        if (round_start) cudaEventDestroy(round_start);
+        if (round_stop) cudaEventDestroy(round_stop);
         cudaStreamDestroy(stream);
     }
 }

@@ -101,8 +101,10 @@ void note_launch();
 void note_launches(uint64_t n);  // kernels run by a replayed CUDA graph
 
 // Exclusive prefix sum of n 32-bit counts into 64-bit offsets (out has n + 1
-// entries; out[n] = total).  Scratch is allocated internally.
-int exclusive_scan_u32_to_u64(const uint32_t *in, uint64_t *out, uint64_t n, cudaStream_t s);
+// entries; out[n] = total).  Scratch is allocated and the stream waited for here,
+// unless the caller keeps a scratch array: then it is grown and nothing is waited for.
+int exclusive_scan_u32_to_u64(const uint32_t *in, uint64_t *out, uint64_t n, cudaStream_t s,
+                              DevArray<uint64_t> *kept = nullptr);
 
 }  // namespace dg
 
@@ -129,12 +131,16 @@ struct dg_graph {
     // Per-round buffers kept between rounds, so a round allocates nothing once
     // the first has run: counters, the visit counts' backup, entropy partial
     // sums, and the walk arena of the last freed dg_paths (largest kept).
-    dg::DevArray<unsigned long long> round_stats;
-    dg::DevArray<uint32_t> round_ctl, freq_backup;
-    dg::DevArray<double> entropy_partial;
+    // A round's counters and the entropy's partial sums lie in one buffer, so that
+    // one copy to page-locked memory and one wait bring all a round reports.
+    dg::DevArray<unsigned long long> round_buf;     // footprints, draws, traces, overflows | queue, longest | partials
+    unsigned long long *round_host = nullptr;       // the same, page-locked
+    cudaEvent_t round_start = nullptr, round_stop = nullptr;
+    dg::DevArray<uint32_t> freq_backup;
     dg::DevArray<uint32_t> spare_verts, spare_lens;
-    dg::DevArray<uint64_t> copy_at;   // dg_paths_copy: walk offsets and compacted walks,
-    dg::DevArray<uint32_t> copy_flat; // kept (and grown) between calls
+    dg::DevArray<uint64_t> copy_at;   // dg_paths_copy: walk offsets, their scan's scratch
+    dg::DevArray<uint64_t> copy_scan; // and compacted walks, kept (and grown) between calls
+    dg::DevArray<uint32_t> copy_flat;
     ~dg_graph();
 };
 

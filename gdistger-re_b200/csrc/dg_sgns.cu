@@ -1420,13 +1420,18 @@ int copy_rows(const dg_sgns *s, bool input, float *host) {
         DG_CUDA(cudaStreamSynchronize(s->stream));
         return DG_OK;
     }
-    dg::DevArray<float> tmp;
-    DG_CUDA(tmp.alloc(n));
-    rows_to_f32<<<dg::sm_count(s->device) * 4, 256, 0, s->stream>>>(input ? s->in_bf.p : s->out_bf.p,
-                                                                     input ? s->in_master.p : s->out_master.p, n,
-                                                                     (uint64_t)s->n_master * s->p.size, tmp.p); dg::note_launch();
-    DG_CUDA(cudaGetLastError());
-    DG_CUDA(cudaMemcpyAsync(host, tmp.p, n * 4, cudaMemcpyDeviceToHost, s->stream));
+    dg::DevArray<float> &tmp = s->out_tmp;
+    if (tmp.n < std::min(n, kOutChunk)) DG_CUDA(tmp.alloc(std::min(n, kOutChunk)));
+    const uint64_t nm = (uint64_t)s->n_master * s->p.size;
+    for (uint64_t at = 0; at < n; at += kOutChunk) {
+        const uint64_t c = std::min(n - at, kOutChunk);
+        rows_to_f32<<<dg::sm_count(s->device) * 4, 256, 0, s->stream>>>(
+            (input ? s->in_bf.p : s->out_bf.p) + at, (input ? s->in_master.p : s->out_master.p) + std::min(at, nm), c,
+            at < nm ? nm - at : 0, tmp.p);
+        dg::note_launch();
+        DG_CUDA(cudaGetLastError());
+        DG_CUDA(cudaMemcpyAsync(host + at, tmp.p, c * 4, cudaMemcpyDeviceToHost, s->stream));
+    }
     DG_CUDA(cudaStreamSynchronize(s->stream));
     return DG_OK;
 }
@@ -1442,6 +1447,7 @@ dg_sgns::~dg_sgns() {
         syn0.release(); syn1.release(); in_bf.release(); out_bf.release(); in_master.release(); out_master.release();
         scratch.release(); queue.release(); stats.release(); adj_in.release(); adj_out.release(); adj_flag.release();
         adj_offs.release(); adj_pin.release(); adj_pout.release(); adj_neg.release(); adj_step.release();
+        out_tmp.release(); pair_ids.release(); pair_loss.release();
         if (adj_exec) cudaGraphExecDestroy(adj_exec);
         cudaStreamDestroy(stream);
     }

@@ -169,6 +169,9 @@ struct AdjStep {
 
 struct dg_sgns;
 namespace dgs {
+// Elements converted and copied to the host at a time: a whole table as FP32 would
+// be as large as the FP32 form's, allocated and freed by every call.
+constexpr uint64_t kOutChunk = 1u << 23;
 // Whether the trainer keeps its rows in FP32 (syn0 / syn1): the word2vec.cu
 // rules; the minibatch and BF16 forms keep BF16 rows + FP32 masters.
 bool fp32_rows(const dg_sgns *s);
@@ -215,5 +218,8 @@ struct dg_sgns {
     dg::DevArray<uint64_t> host_off;     // dg_sgns_train_host: device copies of the caller's walks,
     dg::DevArray<uint32_t> host_verts;   // kept (and grown) between calls
     dg::DevArray<unsigned int> vmax;     // dg_sgns_train_host: largest vertex id of the call
+    mutable dg::DevArray<float> out_tmp; // rows on their way to the host as FP32 (dgs::kOutChunk elements at most)
+    dg::DevArray<uint32_t> pair_ids;     // dg_sgns_loss_grad, _adjoint_step: the caller's ids, kept (and grown)
+    dg::DevArray<double> pair_loss;      // between calls, and the minibatches' losses
     ~dg_sgns();
 };

@@ -490,35 +490,38 @@ int adjoint_run(dg_sgns *s, const dg_sgns_pairs *pp, double *loss) {
     const uint64_t n_batches = (pp->n_pairs + pp->batch - 1) / pp->batch;
     const uint64_t n_neg = n_batches * (uint64_t)pp->negative;
     DG_CHECK(n_neg == 0 || pp->negatives, DG_ERR_ARG, "NULL negatives");
-    for (uint64_t p = 0; p < pp->n_pairs; p++)
-        DG_CHECK(pp->inputs[p] < s->vocab_size && pp->outputs[p] < s->vocab_size, DG_ERR_ARG,
-                 "pair %llu has a row id beyond the vocabulary (%u rows)", (unsigned long long)p, s->vocab_size);
-    for (uint64_t k = 0; k < n_neg; k++)
-        DG_CHECK(pp->negatives[k] < s->vocab_size, DG_ERR_ARG, "negative %llu is beyond the vocabulary (%u rows)",
-                 (unsigned long long)k, s->vocab_size);
+    uint32_t top_pair = 0, top_neg = 0;   // the largest ids: loops the compiler vectorises
+    for (uint64_t p = 0; p < pp->n_pairs; p++) top_pair = std::max(top_pair, std::max(pp->inputs[p], pp->outputs[p]));
+    for (uint64_t k = 0; k < n_neg; k++) top_neg = std::max(top_neg, pp->negatives[k]);
+    if (pp->n_pairs && top_pair >= s->vocab_size)
+        for (uint64_t p = 0; p < pp->n_pairs; p++)
+            DG_CHECK(pp->inputs[p] < s->vocab_size && pp->outputs[p] < s->vocab_size, DG_ERR_ARG,
+                     "pair %llu has a row id beyond the vocabulary (%u rows)", (unsigned long long)p, s->vocab_size);
+    if (n_neg && top_neg >= s->vocab_size)
+        for (uint64_t k = 0; k < n_neg; k++)
+            DG_CHECK(pp->negatives[k] < s->vocab_size, DG_ERR_ARG, "negative %llu is beyond the vocabulary (%u rows)",
+                     (unsigned long long)k, s->vocab_size);
     int rc = adjoint_buffers(s);
     if (rc) return rc;
     const uint64_t n = (uint64_t)s->vocab_size * s->p.size;
-    dg::DevArray<uint32_t> d_in, d_out, d_neg;
-    dg::DevArray<double> d_loss;
-    DG_CUDA(d_in.alloc(pp->n_pairs));
-    DG_CUDA(d_out.alloc(pp->n_pairs));
-    DG_CUDA(d_neg.alloc(n_neg));
-    DG_CUDA(d_loss.alloc(n_batches));
+    const uint64_t n_ids = 2 * pp->n_pairs + n_neg;
+    if (s->pair_ids.n < n_ids) DG_CUDA(s->pair_ids.alloc(n_ids + n_ids / 8));
+    if (s->pair_loss.n < n_batches) DG_CUDA(s->pair_loss.alloc(n_batches + n_batches / 8));
+    uint32_t *d_in = s->pair_ids.p, *d_out = d_in + pp->n_pairs, *d_neg = d_out + pp->n_pairs;
     if (pp->n_pairs) {
-        DG_CUDA(cudaMemcpyAsync(d_in.p, pp->inputs, pp->n_pairs * 4, cudaMemcpyHostToDevice, s->stream));
-        DG_CUDA(cudaMemcpyAsync(d_out.p, pp->outputs, pp->n_pairs * 4, cudaMemcpyHostToDevice, s->stream));
+        DG_CUDA(cudaMemcpyAsync(d_in, pp->inputs, pp->n_pairs * 4, cudaMemcpyHostToDevice, s->stream));
+        DG_CUDA(cudaMemcpyAsync(d_out, pp->outputs, pp->n_pairs * 4, cudaMemcpyHostToDevice, s->stream));
     }
-    if (n_neg) DG_CUDA(cudaMemcpyAsync(d_neg.p, pp->negatives, n_neg * 4, cudaMemcpyHostToDevice, s->stream));
+    if (n_neg) DG_CUDA(cudaMemcpyAsync(d_neg, pp->negatives, n_neg * 4, cudaMemcpyHostToDevice, s->stream));
     DG_CUDA(cudaMemsetAsync(s->adj_in.p, 0, n * 8, s->stream));
     DG_CUDA(cudaMemsetAsync(s->adj_out.p, 0, n * 8, s->stream));
     DG_CUDA(cudaMemsetAsync(s->adj_flag.p, 0, 4, s->stream));
     s->adj_dirty = true;
-    rc = adjoint_grad(s, d_in.p, d_out.p, d_neg.p, pp->n_pairs, pp->batch, pp->negative, d_loss.p);
+    rc = adjoint_grad(s, d_in, d_out, d_neg, pp->n_pairs, pp->batch, pp->negative, s->pair_loss.p);
     if (rc) return rc;
     std::vector<double> bl(n_batches);
     unsigned int flag = 0;
-    if (n_batches) DG_CUDA(cudaMemcpyAsync(bl.data(), d_loss.p, n_batches * 8, cudaMemcpyDeviceToHost, s->stream));
+    if (n_batches) DG_CUDA(cudaMemcpyAsync(bl.data(), s->pair_loss.p, n_batches * 8, cudaMemcpyDeviceToHost, s->stream));
     DG_CUDA(cudaMemcpyAsync(&flag, s->adj_flag.p, 4, cudaMemcpyDeviceToHost, s->stream));
     DG_CUDA(cudaStreamSynchronize(s->stream));
     DG_CHECK(flag == 0, DG_ERR_ARG, "a gradient contribution is not finite or exceeds 2^20 in magnitude");
@@ -646,18 +649,21 @@ extern "C" int dg_sgns_loss_grad(dg_sgns *s, const dg_sgns_pairs *pairs, double 
     if (rc) return rc;
     const uint64_t n = (uint64_t)s->vocab_size * s->p.size;
     if (!grad_in && !grad_out) return DG_OK;
-    dg::DevArray<float> tmp;
-    DG_CUDA(tmp.alloc(n));
+    dg::DevArray<float> &tmp = s->out_tmp;
+    if (tmp.n < std::min(n, dgs::kOutChunk)) DG_CUDA(tmp.alloc(std::min(n, dgs::kOutChunk)));
     for (int k = 0; k < 2; k++) {
         float *host = k == 0 ? grad_in : grad_out;
         if (!host) continue;
-        dgs::adjoint_to_f32<<<dg::sm_count(s->device) * 4, 256, 0, s->stream>>>(k == 0 ? s->adj_in.p : s->adj_out.p,
-                                                                              n, tmp.p);
-        dg::note_launch();
-        DG_CUDA(cudaGetLastError());
-        DG_CUDA(cudaMemcpyAsync(host, tmp.p, n * 4, cudaMemcpyDeviceToHost, s->stream));
-        DG_CUDA(cudaStreamSynchronize(s->stream));
+        for (uint64_t at = 0; at < n; at += dgs::kOutChunk) {
+            const uint64_t c = std::min(n - at, dgs::kOutChunk);
+            dgs::adjoint_to_f32<<<dg::sm_count(s->device) * 4, 256, 0, s->stream>>>(
+                (k == 0 ? s->adj_in.p : s->adj_out.p) + at, c, tmp.p);
+            dg::note_launch();
+            DG_CUDA(cudaGetLastError());
+            DG_CUDA(cudaMemcpyAsync(host + at, tmp.p, c * 4, cudaMemcpyDeviceToHost, s->stream));
+        }
     }
+    DG_CUDA(cudaStreamSynchronize(s->stream));
     return DG_OK;
 }
 

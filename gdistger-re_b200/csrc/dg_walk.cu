@@ -207,10 +207,14 @@ __global__ void __launch_bounds__(THREADS) walk_kernel(WalkArgs a) {
 
 // Per-block partial sums of p_i * (log p_i - log q_i) (walk.hpp:706-725).
 constexpr int kEntropyThreads = 256;
+// words_before: the footprints of earlier rounds; *words: this round's (words_sum of
+// the reference is their sum).
 __global__ void entropy_partials(const uint32_t *__restrict__ deg, const uint32_t *__restrict__ freq, uint32_t v_num,
-                                 double degree_sum, double words_sum, double *partial) {
+                                 double degree_sum, uint64_t words_before, const unsigned long long *words,
+                                 double *partial) {
     __shared__ double red[kEntropyThreads];
     double acc = 0.0;
+    const double words_sum = (double)(words_before + *words);
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < v_num; i += (uint64_t)gridDim.x * blockDim.x) {
         const double pi = (double)deg[i] / degree_sum;
         const double qi = (double)freq[i] / words_sum;
@@ -273,22 +277,6 @@ __global__ void compact_walks(const uint32_t *__restrict__ verts, const uint32_t
     }
 }
 
-int relative_entropy(dg_graph *g, uint64_t words_sum, double *h) {
-    const int blocks = dg::sm_count(g->device) * 4;
-    dg::DevArray<double> &partial = g->entropy_partial;
-    if (partial.n < (size_t)blocks) DG_CUDA(partial.alloc(blocks));
-    entropy_partials<<<blocks, kEntropyThreads, 0, g->stream>>>(g->out_deg.p, g->freq.p, g->v_num, (double)g->m,
-                                                                  (double)words_sum, partial.p); dg::note_launch();
-    DG_CUDA(cudaGetLastError());
-    std::vector<double> host(blocks);
-    DG_CUDA(cudaMemcpyAsync(host.data(), partial.p, blocks * sizeof(double), cudaMemcpyDeviceToHost, g->stream));
-    DG_CUDA(cudaStreamSynchronize(g->stream));
-    double s = 0.0;
-    for (double v : host) s += v;
-    *h = s;
-    return DG_OK;
-}
-
 // One launch of walk_kernel in launch shape I: a persistent grid of as many
 // blocks as fit (each thread pulls walker ids from the queue).
 template <int I>
@@ -319,9 +307,15 @@ int walk_launch(int shape, dg_graph *g, const WalkArgs &a, uint32_t n_walkers) {
     }
 }
 
-// shape < 0: the graph's current (tuned) launch shape.
+// dg_graph::round_buf: four counters, the queue head and the longest walk in one
+// word, three words free, then the entropy's partial sums.
+constexpr size_t kRoundWords = 8;
+
+// shape < 0: the graph's current (tuned) launch shape.  entropy (may be NULL): the
+// relative entropy of the cumulative visits with this round's, formed right behind
+// the walks so that one wait brings both.
 int run_round(dg_graph *g, const dg_walk_params *p, uint32_t round, uint32_t n_walkers, uint32_t stride,
-              std::unique_ptr<dg_paths> &out, int shape = -1) {
+              std::unique_ptr<dg_paths> &out, int shape = -1, double *entropy = nullptr) {
     DG_CHECK(stride >= 2 && stride <= (1u << 16), DG_ERR_ARG, "max_len %u out of range [2, 65536]", stride);
     int rc = dg::ensure_entropy_table(g, stride);
     if (rc) return rc;
@@ -339,12 +333,19 @@ int run_round(dg_graph *g, const dg_walk_params *p, uint32_t round, uint32_t n_w
         DG_CUDA(ps->lens.alloc(n_walkers));
     }
 
-    dg::DevArray<unsigned long long> &stats = g->round_stats;
-    dg::DevArray<uint32_t> &ctl = g->round_ctl;  // [0] queue head, [1] longest walk
-    if (!stats.p) DG_CUDA(stats.alloc(4));
-    if (!ctl.p) DG_CUDA(ctl.alloc(2));
-    DG_CUDA(cudaMemsetAsync(stats.p, 0, 4 * sizeof(unsigned long long), g->stream));
-    DG_CUDA(cudaMemsetAsync(ctl.p, 0, 2 * sizeof(uint32_t), g->stream));
+    const int entropy_blocks = dg::sm_count(g->device) * 4;
+    const size_t words = kRoundWords + (size_t)entropy_blocks;
+    if (g->round_buf.n < words) {
+        DG_CUDA(g->round_buf.alloc(words));
+        if (g->round_host) DG_CUDA(cudaFreeHost(g->round_host));
+        g->round_host = nullptr;
+        DG_CUDA(cudaMallocHost(reinterpret_cast<void **>(&g->round_host), words * 8));
+    }
+    if (!g->round_start) DG_CUDA(cudaEventCreate(&g->round_start));
+    if (!g->round_stop) DG_CUDA(cudaEventCreate(&g->round_stop));
+    unsigned long long *stats = g->round_buf.p;
+    uint32_t *ctl = reinterpret_cast<uint32_t *>(stats + 4);   // [0] queue head, [1] longest walk
+    DG_CUDA(cudaMemsetAsync(stats, 0, kRoundWords * 8, g->stream));
     // Keep the pre-round visit counts so a failed (overflowing) round can be undone.
     dg::DevArray<uint32_t> &freq_backup = g->freq_backup;
     if (freq_backup.n < g->v_num) DG_CUDA(freq_backup.alloc(g->v_num));
@@ -358,9 +359,9 @@ int run_round(dg_graph *g, const dg_walk_params *p, uint32_t round, uint32_t n_w
     a.verts = ps->verts.p;
     a.lens = ps->lens.p;
     a.freq = g->freq.p;
-    a.next = ctl.p;
-    a.stats = stats.p;
-    a.max_len = ctl.p + 1;
+    a.next = ctl;
+    a.stats = stats;
+    a.max_len = ctl + 1;
     a.n_walks = n_walkers;
     a.v_num = g->v_num;
     a.stride = stride;
@@ -369,16 +370,21 @@ int run_round(dg_graph *g, const dg_walk_params *p, uint32_t round, uint32_t n_w
     a.seed_lo = (uint32_t)p->seed;
     a.seed_hi = (uint32_t)(p->seed >> 32);
 
-    dg::EventTimer t;
-    t.start(g->stream);
+    DG_CUDA(cudaEventRecord(g->round_start, g->stream));
     rc = walk_launch(shape < 0 ? g->walk_shape : shape, g, a, n_walkers);
     if (rc) return rc;
-    t.stop(g->stream);
-    unsigned long long h_stats[4];
-    uint32_t h_ctl[2];
-    DG_CUDA(cudaMemcpyAsync(h_stats, stats.p, sizeof(h_stats), cudaMemcpyDeviceToHost, g->stream));
-    DG_CUDA(cudaMemcpyAsync(h_ctl, ctl.p, sizeof(h_ctl), cudaMemcpyDeviceToHost, g->stream));
+    DG_CUDA(cudaEventRecord(g->round_stop, g->stream));
+    if (entropy) {
+        entropy_partials<<<entropy_blocks, kEntropyThreads, 0, g->stream>>>(
+            g->out_deg.p, g->freq.p, g->v_num, (double)g->m, g->visits_total, stats,
+            reinterpret_cast<double *>(stats + kRoundWords));
+        dg::note_launch();
+        DG_CUDA(cudaGetLastError());
+    }
+    DG_CUDA(cudaMemcpyAsync(g->round_host, stats, (entropy ? words : kRoundWords) * 8, cudaMemcpyDeviceToHost, g->stream));
     DG_CUDA(cudaStreamSynchronize(g->stream));
+    const unsigned long long *h_stats = g->round_host;
+    const uint32_t *h_ctl = reinterpret_cast<const uint32_t *>(h_stats + 4);
     if (h_stats[3]) {
         DG_CUDA(cudaMemcpyAsync(g->freq.p, freq_backup.p, (size_t)g->v_num * 4, cudaMemcpyDeviceToDevice, g->stream));
         DG_CUDA(cudaStreamSynchronize(g->stream));
@@ -392,7 +398,15 @@ int run_round(dg_graph *g, const dg_walk_params *p, uint32_t round, uint32_t n_w
     inf.draws = h_stats[1];
     inf.traces = h_stats[2];
     inf.max_len = h_ctl[1];
-    inf.walk_ms = t.ms();
+    float walk_ms = 0.f;
+    DG_CUDA(cudaEventElapsedTime(&walk_ms, g->round_start, g->round_stop));
+    inf.walk_ms = (double)walk_ms;
+    if (entropy) {   // walk.hpp:693-734
+        const double *partial = reinterpret_cast<const double *>(h_stats + kRoundWords);
+        double h = 0.0;
+        for (int k = 0; k < entropy_blocks; k++) h += partial[k];
+        *entropy = h;
+    }
 
     out.swap(ps);
     return DG_OK;
@@ -412,14 +426,10 @@ extern "C" int dg_walk_run_round(dg_graph *g, const dg_walk_params *p, uint32_t 
     const uint32_t stride = p->max_len ? p->max_len : kDefaultStride;
     dg::DeviceGuard guard(g->device);
     std::unique_ptr<dg_paths> ps;
-    int rc = run_round(g, p, round, (uint32_t)n, stride, ps);
+    double h = 0.0;   // relative entropy of cumulative visits vs degree share
+    int rc = run_round(g, p, round, (uint32_t)n, stride, ps, -1, &h);
     if (rc) return rc;
-
-    // Relative entropy of cumulative visits vs degree share (walk.hpp:693-734).
     g->visits_total += ps->info.footprints;
-    double h = 0.0;
-    rc = relative_entropy(g, g->visits_total, &h);
-    if (rc) return rc;
     const double prev = g->entropy_history.empty() ? 0.0 : g->entropy_history.back();
     ps->info.relative_entropy = h;
     ps->info.delta_h = g->entropy_history.empty() ? h : h - prev;
@@ -441,7 +451,7 @@ extern "C" int dg_paths_copy(const dg_paths *ps, uint64_t *offsets, uint32_t *ve
     cudaStream_t s = g->stream;
     dg::DevArray<uint64_t> &at = g->copy_at;
     if (at.n < (size_t)ps->n_walks + 1) DG_CUDA(at.alloc((size_t)ps->n_walks + 1));
-    int rc = dg::exclusive_scan_u32_to_u64(ps->lens.p, at.p, ps->n_walks, s);
+    int rc = dg::exclusive_scan_u32_to_u64(ps->lens.p, at.p, ps->n_walks, s, &g->copy_scan);
     if (rc) return rc;
     if (offsets) DG_CUDA(cudaMemcpyAsync(offsets, at.p, ((size_t)ps->n_walks + 1) * 8, cudaMemcpyDeviceToHost, s));
     if (vertices && ps->info.footprints) {

@@ -15,8 +15,9 @@
 //
 // Here: one 64-bit sort builds the row-sorted CSR, a stable sort of the pairs'
 // unordered keys finds each pair's first occurrence, one warp per first
-// occurrence walks the shorter row and binary-searches the longer one, and the
-// counts are scattered back to input order.
+// occurrence walks the shorter row and looks its elements up in the longer one (a
+// bitmap of the longest rows, a binary search in the others), and the counts are
+// scattered back to input order.
 #include "dg_internal.h"
 
 #include <cub/cub.cuh>
@@ -63,10 +64,69 @@ __device__ __forceinline__ bool in_row(const uint32_t *row, uint64_t len, uint32
     return lo < len && row[lo] == x;
 }
 
+// The longest rows as bitmaps over the vertices: kept to kHubBytes, so that they stay
+// in L2, and to rows of at least 2^kHubLog entries, below which a search is as quick.
+constexpr uint64_t kHubBytes = 64ull << 20;
+constexpr int kHubLog = 7;
+
+struct CnHubs {
+    uint32_t *hist;    // [33] rows by length (floor of log2 + 1); then [33]: shortest length that gets a bitmap, [34]: slots given
+    int32_t *slot;     // [v_num] bitmap of the vertex's row, -1: none
+    uint32_t *bits;    // [slots][words]
+    uint32_t slots, words;
+};
+
+__global__ void cn_lengths(const uint64_t *offsets, uint32_t v_num, CnHubs h) {
+    __shared__ uint32_t count[33];
+    if (threadIdx.x < 33) count[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < v_num; v += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t n = offsets[v + 1] - offsets[v];
+        const int log = n ? min(32, 64 - __clzll((long long)n)) : 0;
+        if (log > kHubLog) atomicAdd(&count[log], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x < 33 && count[threadIdx.x]) atomicAdd(&h.hist[threadIdx.x], count[threadIdx.x]);
+}
+
+// The smallest power of two that at most `slots` rows reach.
+__global__ void cn_pick(CnHubs h) {
+    uint32_t rows = 0;
+    int log = 33;
+    while (log > kHubLog + 1 && rows + h.hist[log - 1] <= h.slots) rows += h.hist[--log];
+    h.hist[33] = log > 32 ? ~0u : 1u << (log - 1);
+}
+
+__global__ void cn_slots(const uint64_t *offsets, uint32_t v_num, CnHubs h) {
+    const uint32_t least = h.hist[33];
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < v_num; v += (uint64_t)gridDim.x * blockDim.x)
+        h.slot[v] = offsets[v + 1] - offsets[v] >= least ? (int32_t)atomicAdd(&h.hist[34], 1u) : -1;
+}
+
+__global__ void cn_bits(const uint64_t *dir, uint64_t m, int bits, CnHubs h) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
+        const int32_t s = h.slot[dir[i] >> bits];
+        if (s < 0) continue;
+        const uint32_t x = (uint32_t)(dir[i] & (((uint64_t)1 << bits) - 1));
+        atomicOr(&h.bits[(uint64_t)s * h.words + (x >> 5)], 1u << (x & 31));
+    }
+}
+
+// Sum over the warp of counts below 2^48.
+__device__ __forceinline__ unsigned long long cn_sum(unsigned long long v) {
+    const uint32_t a = __reduce_add_sync(0xffffffffu, (uint32_t)(v & 0xFFFFFFu));
+    const uint32_t b = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 24));
+    return (unsigned long long)a + ((unsigned long long)b << 24);
+}
+
 // One warp per sorted pair position that starts a group (the pair's first
-// occurrence): the count in that occurrence's orientation.
+// occurrence): the count in that occurrence's orientation.  What bounds it is the
+// probes of the longer rows: the YouTube-shaped graph's 3.25M pairs have 227M
+// elements in their shorter rows, and a binary search each is 2.7G probes of L1 and
+// L2 (5.7 ms).  Two fifths to four fifths of the elements are looked up in the few
+// hundred longest rows, where a bitmap takes one probe (a pass, host to host: 16 -> 11 ms).
 __global__ void cn_count(const uint64_t *pair_sorted, const uint64_t *idx_sorted, uint64_t n, const uint32_t *src,
-                         const uint32_t *dst, const uint64_t *offsets, const uint32_t *nbr, int32_t *cn_sorted) {
+                         const uint32_t *dst, const uint64_t *offsets, const uint32_t *nbr, CnHubs h, int32_t *cn_sorted) {
     const int lane = threadIdx.x & 31;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
@@ -78,33 +138,35 @@ __global__ void cn_count(const uint64_t *pair_sorted, const uint64_t *idx_sorted
         const bool first_long = n1 > n2;                 // gcn.cpp:166-172
         const uint32_t *sh = first_long ? r2 : r1, *lg = first_long ? r1 : r2;
         const uint64_t ns = first_long ? n2 : n1, nl = first_long ? n1 : n2;
+        const int32_t slot = h.slot[first_long ? s : d];
+        const uint32_t *bits = h.bits + (slot < 0 ? 0 : (uint64_t)slot * h.words);
         unsigned long long count = 0, dups = 0, sd = 0;
         uint64_t first = ~0ull;
         if (ns > 0 && nl > 0) {
             for (uint64_t j = lane; j < ns; j += 32) {
                 const uint32_t x = sh[j];
-                if (!in_row(lg, nl, x)) continue;
+                if (slot >= 0 ? !((bits[x >> 5] >> (x & 31)) & 1u) : !in_row(lg, nl, x)) continue;
                 count++;
                 first = min(first, j);
                 if (j > 0 && sh[j - 1] == x) dups++;
                 else if (x == s || x == d) sd++;
             }
         }
-        for (int o = 16; o; o >>= 1) {
-            count += __shfl_xor_sync(0xffffffffu, count, o);
-            dups += __shfl_xor_sync(0xffffffffu, dups, o);
-            sd += __shfl_xor_sync(0xffffffffu, sd, o);
-            first = min(first, (uint64_t)__shfl_xor_sync(0xffffffffu, (unsigned long long)first, o));
+        count = cn_sum(count);
+        if (count == 0) {
+            if (lane == 0) cn_sorted[i] = 0;
+            continue;
         }
+        dups = cn_sum(dups);
+        sd = cn_sum(sd);
+        for (int o = 16; o; o >>= 1) first = min(first, (uint64_t)__shfl_xor_sync(0xffffffffu, (unsigned long long)first, o));
         if (lane == 0) {
             long long c = (long long)count;
-            if (c > 0) {
-                const uint32_t i0 = sh[first];
-                const bool i0_sd = i0 == s || i0 == d;
-                if (i0_sd) c--;
-                // The first element is never a repeat; an s/d first element was taken off above.
-                if (c > 1) c -= (long long)dups + (long long)sd - (i0_sd ? 1 : 0);
-            }
+            const uint32_t i0 = sh[first];
+            const bool i0_sd = i0 == s || i0 == d;
+            if (i0_sd) c--;
+            // The first element is never a repeat; an s/d first element was taken off above.
+            if (c > 1) c -= (long long)dups + (long long)sd - (i0_sd ? 1 : 0);
             cn_sorted[i] = (int32_t)(uint32_t)c;
         }
     }
@@ -170,6 +232,12 @@ extern "C" int dg_common_neighbours(const uint32_t *src, const uint32_t *dst, ui
                  o_dir = part(m * 8), o_dir2 = part(m * 8), o_pair = part(n * 8), o_pair2 = part(n * 8),
                  o_idx = part(n * 8), o_idx2 = part(n * 8), o_sorted = part(n * 4), o_cn = part(n * 4),
                  o_cub = part(cub_bytes ? cub_bytes : 1);
+    CnHubs hubs{};
+    hubs.words = (v_num + 31) / 32;
+    // No more rows than this can have 2^kHubLog entries.
+    hubs.slots = (uint32_t)std::min<uint64_t>(kHubBytes / ((uint64_t)hubs.words * 4), m >> kHubLog);
+    const size_t hub_bytes = (size_t)hubs.slots * hubs.words * 4;
+    const size_t o_hist = part(35 * 4), o_slot = part((size_t)v_num * 4), o_bits = part(hub_bytes);
     dg::DevArray<uint8_t> block;
     DG_CUDA(block.alloc(need));
     uint32_t *const d_src = reinterpret_cast<uint32_t *>(block.p + o_src), *const d_dst = reinterpret_cast<uint32_t *>(block.p + o_dst),
@@ -190,10 +258,21 @@ extern "C" int dg_common_neighbours(const uint32_t *src, const uint32_t *dst, ui
     cn_rows<<<grid, 256, 0, s>>>(dir2, m, v_num, key_bits, offsets, nbr);
     dg::note_launch();
     DG_CUDA(cudaGetLastError());
+    hubs.hist = reinterpret_cast<uint32_t *>(block.p + o_hist);
+    hubs.slot = reinterpret_cast<int32_t *>(block.p + o_slot);
+    hubs.bits = reinterpret_cast<uint32_t *>(block.p + o_bits);
+    DG_CUDA(cudaMemsetAsync(hubs.hist, 0, 35 * 4, s));
+    if (hub_bytes) DG_CUDA(cudaMemsetAsync(hubs.bits, 0, hub_bytes, s));
+    cn_lengths<<<grid, 256, 0, s>>>(offsets, v_num, hubs);
+    cn_pick<<<1, 1, 0, s>>>(hubs);
+    cn_slots<<<grid, 256, 0, s>>>(offsets, v_num, hubs);
+    cn_bits<<<grid, 256, 0, s>>>(dir2, m, key_bits, hubs);
+    dg::note_launches(4);
+    DG_CUDA(cudaGetLastError());
     // Pairs grouped by unordered key, input order kept inside a group (stable sort).
     bytes = cub_bytes;
     DG_CUDA(cub::DeviceRadixSort::SortPairs(block.p + o_cub, bytes, pair, pair2, idx, idx2, n, 0, 2 * key_bits, s));
-    cn_count<<<grid, 256, 0, s>>>(pair2, idx2, n, d_src, d_dst, offsets, nbr, cn_sorted);
+    cn_count<<<grid, 256, 0, s>>>(pair2, idx2, n, d_src, d_dst, offsets, nbr, hubs, cn_sorted);
     dg::note_launch();
     cn_scatter<<<grid, 256, 0, s>>>(pair2, idx2, n, cn_sorted, d_cn);
     dg::note_launch();

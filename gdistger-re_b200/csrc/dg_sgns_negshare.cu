@@ -78,9 +78,10 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int neg = NS == kShareFixedNeg ? kShareFixedNeg : a.negative;
     const uint32_t w = (uint32_t)a.window;
-    // Lanes whose columns are all padding read lane 0's columns, hold context rows of 0 and write nothing.
+    // Lanes whose columns are all padding read and write nothing: every row, sum and
+    // update that they hold is 0.
     const bool own = lane * VEC < (uint32_t)a.used;
-    float *const syn0 = a.syn0 + (own ? lane * VEC : 0), *const syn1 = a.syn1 + (own ? lane * VEC : 0);
+    float *const syn0 = a.syn0 + lane * VEC, *const syn1 = a.syn1 + lane * VEC;
     unsigned long long n_words = 0, n_trained = 0, n_pairs = 0;
     ShareWalk A, B;
     extern __shared__ __align__(16) float share_smem[];   // per walk the centre's row, twice
@@ -119,9 +120,9 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
             return;
         }
     };
-    auto load_context = [&](int32_t word, RowVec<VEC> &r) {
-        load_row<VEC>(syn0 + (size_t)word * D, r);
-        if (!own) zero_row(r);
+    auto load = [&](const float *table, int32_t word, RowVec<VEC> &r) {
+        zero_row(r);
+        if (own) load_row<VEC>(table + (size_t)word * D, r);
     };
 
     for (;;) {
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
             const int32_t word = A.sen[p];
             RowVec<VEC> pos;
             if (A.k == 0) {
-                load_row<VEC>(syn1 + (size_t)word * D, pos);
+                load(syn1, word, pos);
                 share_put(A.pos0, pos);
             } else {
                 share_get(A.pos, pos);
@@ -168,11 +169,11 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
                     const bool two = k + 1 < m;
                     const int32_t w1 = at(k), w2 = two ? at(k + 1) : w1;
                     RowVec<VEC> l1, l2, e, row[NS];
-                    load_context(w1, l1);
-                    load_context(w2, l2);
+                    load(syn0, w1, l1);
+                    load(syn0, w2, l2);
 #pragma unroll
                     for (int j = 0; j < NS; j++)
-                        if (j < neg) load_row<VEC>(syn1 + (size_t)t[j] * D, row[j]);
+                        if (j < neg) load(syn1, t[j], row[j]);
                         else zero_row(row[j]);
                     const float ga = gradients(l1, row);
                     zero_row(e);
@@ -213,13 +214,13 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
                 for (uint32_t c = k; c < min(k + 2, m); c++) {
                     const int32_t w1 = at(c);
                     RowVec<VEC> l1, e;
-                    load_context(w1, l1);
+                    load(syn0, w1, l1);
                     zero_row(e);
                     for (int j = 0; j < neg; j++) {
                         const int32_t tj = A.negs[j];
                         if (tj == word) continue;
                         RowVec<VEC> row;
-                        load_row<VEC>(syn1 + (size_t)tj * D, row);
+                        load(syn1, tj, row);
                         const float g = sg_grad(warp_dot<VEC>(l1, row), 0, a.exp_table, a.alpha);
                         row_fma(e, g, row);
                         if (own) add_row<VEC>(syn1 + (size_t)tj * D, row_mul(g, l1));

@@ -1,6 +1,6 @@
 // Hogwild shared-negative skip-gram on FP32 rows (__sgNegReuse, word2vec.cu:231-303),
 // two pairs at a time: the form of DG_SGNS_SG_SHARED that trains walks of at most
-// 64 tokens with rows of 64 to 256 columns and up to eight negatives
+// 64 tokens with rows of 64 to 256 columns and three to five negatives
 // (sgns_negshare_kernel, dg_sgns_w2v.cu, trains the others and the deterministic
 // runs).
 //
@@ -17,8 +17,19 @@
 // sgns_negshare_kernel's hold two walks each and train two pairs of either in turn.
 //
 // A round of the 50,000-vertex graph at size 200, window 5, negative 5, with its
-// read-back: 20.5 -> 11.6 ms.  The rows end 1.1 to 1.5 times as far from the one-pair
-// kernel's as two equal runs of that kernel from each other.
+// read-back: 21.2 -> 12.1 ms.
+//
+// Why three to five negatives.  Each negative row is read once for two pairs, so it
+// misses the updates of about twice as many pairs of other walks, and its share of a
+// walk's updates grows with their number: on graphs of 10,000 to 200,000 vertices, sizes
+// 64 to 256, the rows end 1.0 to 1.6 times as far (2.0 at 200 columns and three
+// negatives, once) from the one-pair kernel's as two equal runs of that kernel from each
+// other with three to five negatives, but up to 3.0 times with seven and 2.5 with eight
+// (64 columns the worst; single values leave what that kernel's own runs show).  Below
+// three there is too little to share: 40,000 vertices, size 64, window 8 takes 3.9 ms
+// against 3.3 with one negative, 120,000 at size 128, window 5 10.6 against 10.7 with
+// two, while three (40,000, size 64, window 10) take 4.8 against 5.4 and four (200,000,
+// size 100, window 6) 20.6 against 26.8.
 #include "dg_sgns.h"
 #include "dg_sgns_dev.cuh"
 
@@ -28,8 +39,8 @@ namespace dgs {
 
 constexpr int kShareWarps = 8;             // warps of a block
 constexpr uint32_t kShareTokens = 64;      // the longest walk of this kernel
-constexpr int kShareFixedNeg = 5;
-constexpr int kSharePairNeg = 8;           // the largest negative count of this kernel
+constexpr int kShareLeastNeg = 3;          // the negative counts of this kernel
+constexpr int kShareMostNeg = 5;
 
 // Blocks per SM: two walks a warp, 32 walks up to 128 columns, 16 at 256.
 constexpr int share_pair_blocks(int vec) { return vec <= 4 ? 2 : 1; }
@@ -66,9 +77,9 @@ __device__ __forceinline__ void share_get(const float *p, RowVec<VEC> &r) {
     }
 }
 
-// Lane l owns columns [l * VEC, l * VEC + VEC) of every row.  NS: the negatives at
-// compile time (5), or up to 8 read from a.negative.
-template <int VEC, int NS>
+// Lane l owns columns [l * VEC, l * VEC + VEC) of every row.  FIXED: NS negatives
+// (word2vec's default), else up to NS, read from a.negative.
+template <int VEC, int NS, bool FIXED>
 __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
     sgns_negshare_pair_kernel(SgnsArgs a, WalkSet ws, uint32_t walks) {
     constexpr int D = 32 * VEC, M = pow2_at_least(NS + 1), GROUP = 32 / M;
@@ -76,7 +87,7 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
     __shared__ int32_t sen_all[kShareWarps][2][kShareTokens];
     __shared__ int32_t negs_all[kShareWarps][2][NS];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int neg = NS == kShareFixedNeg ? kShareFixedNeg : a.negative;
+    const int neg = FIXED ? NS : a.negative;
     const uint32_t w = (uint32_t)a.window;
     // Lanes whose columns are all padding read and write nothing: every row, sum and
     // update that they hold is 0.
@@ -259,12 +270,12 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
 
 bool negshare_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
     return !s->p.deterministic && ws.max_len > 0 && ws.max_len <= kShareTokens && s->p.size >= 64 && s->p.size <= 256 &&
-           a.negative <= kSharePairNeg && a.vocab_size > 1;
+           a.negative >= kShareLeastNeg && a.negative <= kShareMostNeg && a.vocab_size > 1;
 }
 
-template <int V, int NS>
+template <int V, int NS, bool FIXED>
 static int negshare_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    auto kern = sgns_negshare_pair_kernel<V, NS>;
+    auto kern = sgns_negshare_pair_kernel<V, NS, FIXED>;
     const uint32_t want = s->p.workers;   // the caller's bound on walks under way: a warp each, or two if need be
     const int warps = want > 0 && want < (uint32_t)kShareWarps ? (int)want : kShareWarps;
     int per_sm = 0;
@@ -282,8 +293,8 @@ static int negshare_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws
 
 template <int V>
 static int negshare_pair_size(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    return a.negative == kShareFixedNeg ? negshare_pair_launch<V, kShareFixedNeg>(s, a, ws)
-                                        : negshare_pair_launch<V, kSharePairNeg>(s, a, ws);
+    return a.negative == kShareMostNeg ? negshare_pair_launch<V, kShareMostNeg, true>(s, a, ws)
+                                       : negshare_pair_launch<V, kShareMostNeg, false>(s, a, ws);
 }
 
 int launch_negshare_pair(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {

@@ -1,33 +1,45 @@
 // Hogwild CBOW on FP32 rows (cbow_kernel, word2vec.cu:401-509), two centres at a
-// time: the form of DG_SGNS_CBOW that trains walks of at most 32 tokens
-// (sgns_cbow_kernel, dg_sgns_w2v.cu, trains longer ones, rows of 512, more than
-// eight negatives and the one-warp deterministic runs).
+// time: the form of DG_SGNS_CBOW that trains walks of at most 32 tokens with rows
+// of up to 128 columns and up to five negatives, or, with hierarchical softmax, up
+// to 256 columns and eight negatives (sgns_cbow_kernel, dg_sgns_w2v.cu, trains the
+// others and the one-warp deterministic runs).
 //
 // What bounds the rule is the L2's reduction rate.  A centre with cw contexts and
 // n negatives reads cw + 1 + n rows and adds to as many; on rows that L2 holds, a
 // B200 reads 18.1 TB/s of 512-byte rows but reduces into them at 5.9 TB/s (a
-// vector atomic and a bulk reduction alike), and the two times add up: 9 contexts
-// and 6 targets cost 15 x 512 B x (1 / 18.1 + 1 / 5.9) = 1.7 ns a centre, which was
-// the time of the kernel that trains one centre at a time (1.75 ns a token).  The
-// windows of two neighbouring centres are nearly the same rows, so here a warp
-// reads the rows of both at once and each row receives the sum of both centres'
-// e in one atomic: 6 row reads and reductions a centre for the contexts, not 9.
+// vector atomic and a bulk reduction alike).  9 contexts and 6 targets are 1.30 ns
+// of reductions and 0.42 ns of reads a centre; the kernel that trains one centre at
+// a time takes 1.75.  The windows of two neighbouring centres are nearly the same
+// rows, so here a warp reads the rows of both at once and each row receives the sum
+// of both centres' e in one atomic: 6.2 row reads and reductions a centre for the
+// contexts, not 9.
 //
 // Measured on a B200, size 128, window 10, negative 5: a YouTube-shaped round
 // (25.0M tokens) in 33.0 ms instead of 43.8; a round of the 10,000-vertex graph
 // at size 100, whose padding columns are no longer moved, in 0.38 ms instead of
-// 0.54.  What bounds it now: the same L2 reductions (12 rows a centre, 1.36 ns of
-// 1.32 ns a token), then DRAM (5 KB a token, 0.76 ns).
+// 0.54.  What bounds it now: the same L2 reductions (12.2 rows a centre, 1.06 ns of
+// 1.32 ns a token; its reads are 0.35 ns more where the two do not overlap), then
+// DRAM (5 KB a token, 0.76 ns).
 //
-// Larger groups would save more (four centres: 8.06 ms for 300,000 walks, two:
-// 9.3), but a Hogwild run's rows depend on how many updates are under way unseen
-// and on how many walks are trained at once: with one of the two doubled or
-// halved, the rows of a 10,000-vertex round end 3 to 4 times further from the
-// one-centre kernel's than two equal runs of that kernel from each other.  So
-// 16 warps of an SM train two centres each, where sgns_cbow_kernel's 32 train
-// one, and each holds two walks that it trains in turn: 32 walks, 32 centres
-// under way (8 of each at 256 columns, where a warp holds one walk and eight
-// warps fit).  The rows then differ 1.4 to 1.7 times as far as two equal runs.
+// A Hogwild run's rows depend on how many updates are under way unseen and on how
+// many walks are trained at once.  So 16 warps of an SM train two centres each,
+// where sgns_cbow_kernel's 32 train one, and each holds two walks that it trains in
+// turn: 32 walks, 32 centres under way.  Measured against sgns_cbow_kernel's rows,
+// over the distance of two equal runs of that kernel (graphs of 10,000 to 1.1M
+// vertices, windows 1 to 10, a job's last learning rate):
+//   columns   negatives   input rows   output rows
+//   32..128   0..5        1.1 .. 2.4   1.0 .. 1.7
+//   32..128   7, 8        1.8 .. 2.5   1.5 .. 1.9
+//   200, 256  3..8        1.7 .. 7.2   1.3 .. 4.4    (no hierarchical softmax)
+//   64..256   3..8, HS    0.9 .. 1.8   0.9 .. 1.3
+// Hence the rule: at 256 columns sgns_cbow_kernel's registers leave it eight warps, so
+// eight warps of two centres have twice as many under way; and with more negatives
+// than five single values end further off than that kernel's own runs show.  With
+// hierarchical softmax the updates of the rows near the root outweigh all that, and
+// both kernels' runs differ alike.
+// Other schedules were further off: 14 or 12 warps of 16 (up to 4.9 and 6.0), targets
+// read in groups of two to four after the contexts (up to 3.0, and 5 to 15 % slower at
+// 64 columns), four centres at a time (8.06 ms for 300,000 walks, two: 9.3).
 #include "dg_sgns.h"
 #include "dg_sgns_dev.cuh"
 
@@ -37,8 +49,9 @@ namespace dgs {
 
 constexpr int kCbowWarps = 8;             // warps of a block
 constexpr uint32_t kCbowMaxTokens = 32;   // a lane per token
-constexpr int kCbowFixedNeg = 5;
-constexpr int kCbowPairNeg = 8;           // the largest negative count of this kernel
+constexpr int kCbowPairNeg = 5;           // the largest negative count of this kernel
+constexpr int kCbowPairHsNeg = 8;         // the same with hierarchical softmax
+constexpr int kCbowPairSize = 128;        // the largest row without it
 
 constexpr int cbow_pair_walks(int vec) { return vec <= 4 ? 2 : 1; }    // walks that a warp trains in turn
 constexpr int cbow_pair_blocks(int vec) { return vec <= 4 ? 2 : 1; }   // blocks per SM
@@ -86,7 +99,7 @@ struct CbowWalk {
 // warp's own updates are all seen.  Target rows are read when their centre
 // starts, after the reductions of the centre before.
 //
-// NS: the negatives at compile time (5), or up to 8 read from a.negative.
+// FIXED: NS negatives (5, word2vec's default), else up to NS, read from a.negative.
 //
 // HS: hierarchical softmax over the centre's Huffman path before its targets
 // (word2vec.cu:436-455; hs_path, dg_sgns_dev.cuh).  Every path runs through the
@@ -98,7 +111,7 @@ struct CbowWalk {
 // each another slice's, and a path's nodes are read four at a time.
 // A round of the 50,000-vertex graph, size 128, window 5, with its read-back:
 // 11.4 -> 7.2 ms.
-template <int VEC, int NS, bool HS>
+template <int VEC, int NS, bool FIXED, bool HS>
 __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
     sgns_cbow_pair_kernel(SgnsArgs a, WalkSet ws, uint32_t walks, float *hot, int32_t hot_from) {
     constexpr int D = 32 * VEC, M = pow2_at_least(NS + 1), GROUP = 32 / M;
@@ -107,7 +120,7 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
     __shared__ __align__(16) int32_t sen_all[kCbowWarps][2][kCbowMaxTokens];
     __shared__ int32_t negs_all[kCbowWarps][2][kCbowMaxTokens * NS];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int neg = NS == kCbowFixedNeg ? kCbowFixedNeg : a.negative;
+    const int neg = FIXED ? NS : a.negative;
     const uint32_t w = (uint32_t)a.window;
     // Lanes whose columns are all padding (a size such as 100 or 200, stored with
     // the next power of two) read lane 0's columns, hold x = 0 and write nothing.
@@ -360,12 +373,13 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
 
 bool cbow_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
     return s->p.mode == DG_SGNS_CBOW && !s->p.deterministic && ws.max_len > 0 && ws.max_len <= kCbowMaxTokens &&
-           s->p.size <= 256 && a.negative <= kCbowPairNeg && a.vocab_size > 1;
+           s->p.size <= (a.hs ? 256 : kCbowPairSize) && a.negative <= (a.hs ? kCbowPairHsNeg : kCbowPairNeg) &&
+           a.vocab_size > 1;
 }
 
-template <int V, int NS, bool HS>
+template <int V, int NS, bool FIXED, bool HS>
 static int cbow_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    auto kern = sgns_cbow_pair_kernel<V, NS, HS>;
+    auto kern = sgns_cbow_pair_kernel<V, NS, FIXED, HS>;
     const uint32_t want = s->p.workers;   // the caller's bound on walks under way: a warp each, or two if need be
     const int warps = want > 0 && want < (uint32_t)kCbowWarps ? (int)want : kCbowWarps;
     int per_sm = 0;
@@ -391,14 +405,18 @@ static int cbow_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
     return DG_OK;
 }
 
+template <int V, bool HS>
+static int cbow_pair_negatives(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
+    if (HS && a.negative > kCbowPairNeg) return cbow_pair_launch<V, HS ? kCbowPairHsNeg : kCbowPairNeg, false, HS>(s, a, ws);
+    return a.negative == kCbowPairNeg ? cbow_pair_launch<V, kCbowPairNeg, true, HS>(s, a, ws)
+                                      : cbow_pair_launch<V, kCbowPairNeg, false, HS>(s, a, ws);
+}
+
 template <int V>
 static int cbow_pair_size(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    const bool fixed = a.negative == kCbowFixedNeg;
-    if (a.hs)
-        return fixed ? cbow_pair_launch<V, kCbowFixedNeg, true>(s, a, ws)
-                     : cbow_pair_launch<V, kCbowPairNeg, true>(s, a, ws);
-    return fixed ? cbow_pair_launch<V, kCbowFixedNeg, false>(s, a, ws)
-                 : cbow_pair_launch<V, kCbowPairNeg, false>(s, a, ws);
+    if (a.hs) return cbow_pair_negatives<V, true>(s, a, ws);
+    if constexpr (32 * V <= kCbowPairSize) return cbow_pair_negatives<V, false>(s, a, ws);
+    return dg::fail(DG_ERR_STATE, "rows of %d columns are not trained two centres at a time", 32 * V);
 }
 
 int launch_cbow_pair(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {

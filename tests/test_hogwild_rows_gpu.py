@@ -59,3 +59,11 @@ def _ratios(corpus, **kw):
     (64, 8, 3, 4), (128, 5, 5, 4), (200, 10, 5, 4), (64, 7, 7, 1.5), (64, 9, 8, 1.5), (256, 5, 7, 1.5), (128, 5, 2, 1.5)])
 def test_shared_negatives(corpus, size, window, negative, most):
     assert max(_ratios(corpus, mode="sg_shared", size=size, window=window, negative=negative)) <= most
+
+
+@pytest.mark.parametrize("size,window,negative,hs,most", [
+    (32, 6, 5, False, 4), (64, 10, 3, False, 4), (100, 8, 5, False, 4), (128, 5, 1, False, 4), (128, 9, 5, True, 4),
+    (64, 8, 8, True, 4), (256, 7, 3, True, 4), (200, 9, 5, False, 1.5), (256, 5, 5, False, 1.5), (64, 9, 8, False, 1.5),
+    (128, 10, 7, False, 1.5)])
+def test_cbow(corpus, size, window, negative, hs, most):
+    assert max(_ratios(corpus, mode="cbow", size=size, window=window, negative=negative, hs=hs)) <= most

@@ -1,0 +1,72 @@
+"""The CBOW pair kernel (dg_sgns_cbow.cu) run by one warp, measured against what a run
+changes, and both pair kernels with two walks to a warp.
+
+One warp: as test_negshare_updates_gpu.py, the difference from the sequential run relative
+to the update, on walks that step back (the windows of neighbouring centres then hold one
+word several times).  A sum that rounds across a boundary of the sigmoid table changes one
+of some 960 terms by 0.003 / 0.5, 1.9e-4 of the update at most; the bound, 4e-4, allows for
+two.  With hierarchical softmax the change also moves the root's row, which enters every
+later centre: a NumPy model of the rule shows up to 4.0e-4 for one crossing in 120 runs
+(5e-7 without); the bound there is 2e-3.  In that model the rows are 1.3e-2 off (7.9e-2 with
+hierarchical softmax) where the second centre's mean misses the first one's update.
+
+Two walks: more walks than warps, each of words that no other walk holds, so that only the
+negatives' rows are shared; at this learning rate runs whose walks see none or all of each
+other's updates differ by 4.4e-4 of the update (the same model).  A warp that took one
+walk's words, negatives or kept row for the other's would be off by the whole update; the
+bound is 5e-3."""
+import numpy as np
+import pytest
+
+from distger.sgns import SGNS
+
+pytestmark = pytest.mark.gpu
+V = 60
+
+
+def _of_the_update(rows, want, init):
+    return float(np.linalg.norm(rows.astype(np.float64) - want) / np.linalg.norm(want.astype(np.float64) - init))
+
+
+def _both(offs, verts, counts, init, others, **kw):
+    got = []
+    for more in (dict(deterministic=True), others):
+        s = SGNS(counts.size, counts, sample=0, min_count=0, seed=5, **more, **kw)
+        s.set_rows(*init)
+        s.train_host(offs, verts)
+        got.append((s.embedding(), s.output_rows()))
+        s.close()
+    (i0, ids0), o0 = got[0]
+    (i1, ids1), o1 = got[1]
+    np.testing.assert_array_equal(ids0, ids1)
+    return _of_the_update(i1, i0, init[0]), _of_the_update(o1, o0, init[1])
+
+
+def _init(n, size):
+    rng = np.random.default_rng(2)
+    return [rng.normal(size=(n, size)).astype(np.float32) * np.float32(0.3) for _ in range(2)]
+
+
+@pytest.mark.parametrize("hs", [False, True])
+@pytest.mark.parametrize("negative", [0, 3, 5, 8])
+@pytest.mark.parametrize("size", [32, 64, 65, 100, 128, 200, 256])
+def test_one_warp_makes_the_sequential_update(distger_lib, size, negative, hs):
+    rng = np.random.default_rng(size)
+    walks = rng.integers(0, V, size=(10, 16))
+    walks[::2, 2::2] = walks[::2, :1]
+    walks[1::2, 3::4] = walks[1::2, 1::4]
+    counts = np.random.default_rng(1).integers(1, 200, size=V).astype(np.uint32)
+    off = _both((np.arange(11) * 16).astype(np.uint64), walks.ravel().astype(np.uint32), counts, _init(V, size),
+                dict(workers=1), size=size, window=5, negative=negative, alpha=0.05, table_size=100_000, mode="cbow", hs=hs)
+    assert max(off) < (2e-3 if hs else 4e-4)
+
+
+@pytest.mark.parametrize("mode,size,negative", [("cbow", 64, 5), ("cbow", 100, 3), ("cbow", 128, 5), ("sg_shared", 64, 5),
+                                                ("sg_shared", 128, 3), ("sg_shared", 200, 5)])
+def test_two_walks_to_a_warp(distger_lib, mode, size, negative):
+    n, length = 6000, 8
+    words = np.random.default_rng(4).permutation(n * length).astype(np.uint32)
+    off = _both((np.arange(n + 1) * length).astype(np.uint64), words, np.full(n * length, 10, np.uint32),
+                _init(n * length, size), {}, size=size, window=10, negative=negative,
+                alpha=5e-4 if mode == "cbow" else 5e-5, table_size=1_000_000, mode=mode)
+    assert max(off) < 5e-3

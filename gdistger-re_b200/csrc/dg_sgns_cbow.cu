@@ -40,6 +40,7 @@
 // Other schedules were further off: 14 or 12 warps of 16 (up to 4.9 and 6.0), targets
 // read in groups of two to four after the contexts (up to 3.0, and 5 to 15 % slower at
 // 64 columns), four centres at a time (8.06 ms for 300,000 walks, two: 9.3).
+#include "dg_pair_grid.h"
 #include "dg_sgns.h"
 #include "dg_sgns_dev.cuh"
 
@@ -380,13 +381,10 @@ bool cbow_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
 template <int V, int NS, bool FIXED, bool HS>
 static int cbow_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
     auto kern = sgns_cbow_pair_kernel<V, NS, FIXED, HS>;
-    const uint32_t want = s->p.workers;   // the caller's bound on walks under way: a warp each, or two if need be
-    const int warps = want > 0 && want < (uint32_t)kCbowWarps ? (int)want : kCbowWarps;
     int per_sm = 0;
-    DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, 0));
-    int blocks = std::min(std::max(per_sm, 1), cbow_pair_blocks(V)) * dg::sm_count(s->device);
-    const uint32_t walks = want > 0 && want <= (uint32_t)(blocks * warps) ? 1u : (uint32_t)cbow_pair_walks(V);
-    if (want > 0) blocks = std::min(blocks, std::max(1, (int)(want / (walks * (uint32_t)warps))));
+    DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kCbowWarps, 0));
+    const PairGrid g = pair_grid(s->p.workers, {std::min(std::max(per_sm, 1), cbow_pair_blocks(V)) * dg::sm_count(s->device),
+                                                kCbowWarps, (uint32_t)cbow_pair_walks(V)});
     // The last rows of the table: inner nodes are rows 0 .. vocabulary - 2, the root the last of them.
     const uint32_t n_hot = HS ? std::min(kHotNodes, s->vocab_size) : 0;
     const int32_t hot_from = HS ? (int32_t)(s->vocab_size - n_hot) : 0;
@@ -395,7 +393,7 @@ static int cbow_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
         cbow_hot_rows<V><<<n_hot, 32, 0, s->stream>>>(s->syn1.p, s->hs_hot.p, hot_from, true);
         dg::note_launch();
     }
-    kern<<<blocks, 32 * warps, 0, s->stream>>>(a, ws, walks, s->hs_hot.p, hot_from);
+    kern<<<g.blocks, 32 * g.warps, 0, s->stream>>>(a, ws, g.walks, s->hs_hot.p, hot_from);
     dg::note_launch();
     if (HS) {
         cbow_hot_rows<V><<<n_hot, 32, 0, s->stream>>>(s->syn1.p, s->hs_hot.p, hot_from, false);

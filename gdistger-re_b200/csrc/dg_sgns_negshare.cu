@@ -30,6 +30,7 @@
 // against 3.3 with one negative, 120,000 at size 128, window 5 10.6 against 10.7 with
 // two, while three (40,000, size 64, window 10) take 4.8 against 5.4 and four (200,000,
 // size 100, window 6) 20.6 against 26.8.
+#include "dg_pair_grid.h"
 #include "dg_sgns.h"
 #include "dg_sgns_dev.cuh"
 
@@ -276,16 +277,13 @@ bool negshare_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &w
 template <int V, int NS, bool FIXED>
 static int negshare_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
     auto kern = sgns_negshare_pair_kernel<V, NS, FIXED>;
-    const uint32_t want = s->p.workers;   // the caller's bound on walks under way: a warp each, or two if need be
-    const int warps = want > 0 && want < (uint32_t)kShareWarps ? (int)want : kShareWarps;
     int per_sm = 0;
-    const size_t smem = (size_t)warps * 4 * 32 * V * sizeof(float);
+    const size_t smem = (size_t)kShareWarps * 4 * 32 * V * sizeof(float);
     DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem));
-    int blocks = std::min(std::max(per_sm, 1), share_pair_blocks(V)) * dg::sm_count(s->device);
-    const uint32_t walks = want > 0 && want <= (uint32_t)(blocks * warps) ? 1u : 2u;
-    if (want > 0) blocks = std::min(blocks, std::max(1, (int)(want / (walks * (uint32_t)warps))));
-    kern<<<blocks, 32 * warps, smem, s->stream>>>(a, ws, walks);
+    DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kShareWarps, smem));
+    const PairGrid g = pair_grid(s->p.workers, {std::min(std::max(per_sm, 1), share_pair_blocks(V)) * dg::sm_count(s->device),
+                                                kShareWarps, 2});
+    kern<<<g.blocks, 32 * g.warps, smem / kShareWarps * g.warps, s->stream>>>(a, ws, g.walks);
     dg::note_launch();
     DG_CUDA(cudaGetLastError());
     return DG_OK;

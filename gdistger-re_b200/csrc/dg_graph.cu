@@ -258,6 +258,7 @@ int ensure_entropy_table(dg_graph *g, uint32_t max_sn) {
         }
         st[s] = double4{hi, lo, ES, ESS - ES * ES};
     }
+    g->etable_max_sn = 0;   // until both tables are filled
     DG_CUDA(g->etable.alloc(n));
     DG_CUDA(g->step_table.alloc(st.size()));
     DG_CUDA(cudaMemcpyAsync(g->etable.p, t.data(), n * 8, cudaMemcpyHostToDevice, g->stream));

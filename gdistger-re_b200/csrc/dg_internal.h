@@ -42,11 +42,15 @@ struct DevArray {
         p = nullptr;
         n = 0;
     }
+    // Where the allocation is refused the array is empty (p null, n 0), so that a caller
+    // that keeps it and grows it by n asks again the next time.
     cudaError_t alloc(size_t count) {
         release();
-        n = count;
         if (count == 0) return cudaSuccess;
-        return cudaMalloc(reinterpret_cast<void **>(&p), count * sizeof(T));
+        const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&p), count * sizeof(T));
+        if (e == cudaSuccess) n = count;
+        else p = nullptr;
+        return e;
     }
     size_t bytes() const { return n * sizeof(T); }
     void swap(DevArray &o) {

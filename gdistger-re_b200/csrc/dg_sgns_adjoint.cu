@@ -454,7 +454,7 @@ AdjArgs adjoint_args(dg_sgns *s, const uint32_t *inputs, const uint32_t *outputs
 
 int adjoint_buffers(dg_sgns *s) {
     const uint64_t n = (uint64_t)s->vocab_size * s->p.size;
-    if (s->adj_in.n != n) {
+    if (s->adj_in.n != n || s->adj_out.n != n) {
         DG_CUDA(s->adj_in.alloc(n));
         DG_CUDA(s->adj_out.alloc(n));
         s->adj_dirty = true;

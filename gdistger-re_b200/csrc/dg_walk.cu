@@ -335,11 +335,13 @@ int run_round(dg_graph *g, const dg_walk_params *p, uint32_t round, uint32_t n_w
 
     const int entropy_blocks = dg::sm_count(g->device) * 4;
     const size_t words = kRoundWords + (size_t)entropy_blocks;
-    if (g->round_buf.n < words) {
+    if (g->round_buf.n < words || !g->round_host) {
         DG_CUDA(g->round_buf.alloc(words));
         if (g->round_host) DG_CUDA(cudaFreeHost(g->round_host));
         g->round_host = nullptr;
-        DG_CUDA(cudaMallocHost(reinterpret_cast<void **>(&g->round_host), words * 8));
+        void *page_locked = nullptr;
+        DG_CUDA(cudaMallocHost(&page_locked, words * 8));
+        g->round_host = static_cast<unsigned long long *>(page_locked);
     }
     if (!g->round_start) DG_CUDA(cudaEventCreate(&g->round_start));
     if (!g->round_stop) DG_CUDA(cudaEventCreate(&g->round_stop));

@@ -124,7 +124,8 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
     const int neg = FIXED ? NS : a.negative;
     const uint32_t w = (uint32_t)a.window;
     // Lanes whose columns are all padding (a size such as 100 or 200, stored with
-    // the next power of two) read lane 0's columns, hold x = 0 and write nothing.
+    // the next power of two) read lane 0's columns, hold x = 0, give 0 to every sum
+    // (0 times an infinity would be no number) and write nothing.
     const bool own = lane * VEC < (uint32_t)a.used;
     float *const syn0 = a.syn0 + (own ? lane * VEC : 0), *const syn1 = a.syn1 + (own ? lane * VEC : 0);
     // This lane's columns of output row `id`.
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
         if (!(fl & 0x80000000u)) {   // all sums and gradients at once
             float f[M];
 #pragma unroll
-            for (int j = 0; j < M; j++) f[j] = j <= NS && j <= neg ? row_dot(x, q.row[j <= NS ? j : 0]) : 0.f;
+            for (int j = 0; j < M; j++) f[j] = j <= NS && j <= neg && own ? row_dot(x, q.row[j <= NS ? j : 0]) : 0.f;
             const float mine = warp_sums_split<M>(f, lane);
             const uint32_t jm = lane / GROUP;
             const float gm = (fl >> jm) & 1u ? sg_grad(mine, jm == 0, a.exp_table, a.alpha) : 0.f;
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
 #pragma unroll
             for (int j = 0; j <= NS; j++) {
                 if (!((fl >> j) & 1u)) continue;
+                if (!own) zero_row(q.row[j]);
                 const float g = sg_grad(warp_dot<VEC>(x, q.row[j]), j == 0, a.exp_table, a.alpha);
                 row_fma(e, g, q.row[j]);
                 const RowVec<VEC> upd = row_mul(g, x);
@@ -236,13 +238,13 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
         }
     };
     // x / cw, correctly rounded from the rounded reciprocal (Markstein 1990):
-    // q = x r, then q + (x - q cw) r.  Padding lanes become 0.
+    // q = x r, then q + (x - q cw) r; infinities stay as they are.  Padding lanes become 0.
     auto mean = [&](RowVec<VEC> &x, uint32_t window) {
         const float cw = (float)__popc(window), r = __frcp_rn(cw);
 #pragma unroll
         for (int i = 0; i < VEC; i++) {
             const float q = x.v[i] * r;
-            x.v[i] = own ? fmaf(fmaf(-q, cw, x.v[i]), r, q) : 0.f;
+            x.v[i] = !own ? 0.f : fabsf(q) < INFINITY ? fmaf(fmaf(-q, cw, x.v[i]), r, q) : q;
         }
     };
 
@@ -268,7 +270,7 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
                 else zero_row(row[j]);
             }
 #pragma unroll
-            for (int j = 0; j < H; j++) f[j] = row_dot(x, row[j]);
+            for (int j = 0; j < H; j++) f[j] = own ? row_dot(x, row[j]) : 0.f;
             const float mine = warp_sums_split<H>(f, lane);
             const float lab = __shfl_sync(kAll, label, lane / (32 / H));
             const bool skip = mine <= -kMaxExp || mine >= kMaxExp;
@@ -332,7 +334,7 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
             if (wq) {
                 if (!HS) load_targets(p + 1, q);
                 const int pairs = __reduce_add_sync(kAll, ((wq >> lane) & 1u) ? __popc(A.same & wp) : 0);
-                row_fma(y, (float)pairs, e);
+                if (pairs) row_fma(y, (float)pairs, e);   // 0 of an infinite e would be no number
                 mean(y, wq);
                 zero_row(x);   // from here the second centre's e
                 if (HS) {

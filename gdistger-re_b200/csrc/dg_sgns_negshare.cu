@@ -191,7 +191,8 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
                     zero_row(e);
 #pragma unroll
                     for (int j = 0; j < NS; j++) {
-                        const float g = __shfl_sync(kAll, ga, j * GROUP);   // 0 where the negative does not train
+                        const float g = __shfl_sync(kAll, ga, j * GROUP);
+                        if (!((live >> j) & 1u)) continue;
                         row_fma(e, g, row[j]);
                         if (two) row_fma(row[j], g, l1);
                     }
@@ -207,7 +208,10 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
                         gb = gradients(l2, row);
                         zero_row(e);
 #pragma unroll
-                        for (int j = 0; j < NS; j++) row_fma(e, __shfl_sync(kAll, gb, j * GROUP), row[j]);
+                        for (int j = 0; j < NS; j++) {
+                            const float g = __shfl_sync(kAll, gb, j * GROUP);
+                            if ((live >> j) & 1u) row_fma(e, g, row[j]);
+                        }
                         const float g = __shfl_sync(kAll, gb, NS * GROUP);
                         row_fma(e, g, pos);
                         row_fma(pos, g, l2);
@@ -218,7 +222,7 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
                         const float g1 = __shfl_sync(kAll, ga, j * GROUP), g2 = __shfl_sync(kAll, gb, j * GROUP);
                         if (!((live >> j) & 1u)) continue;
                         RowVec<VEC> upd = row_mul(g1, l1);
-                        row_fma(upd, g2, l2);
+                        if (two) row_fma(upd, g2, l2);
                         if (own) add_row<VEC>(syn1 + (size_t)t[j] * D, upd);
                     }
                 }

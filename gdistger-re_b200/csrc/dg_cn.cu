@@ -28,8 +28,7 @@
 namespace {
 
 // Keys of two ids in 2 * bits bits: the sorts pass over no others.
-__global__ void cn_keys(const uint32_t *src, const uint32_t *dst, uint64_t n, int undirected, int bits, uint64_t *dir,
-                        uint64_t *pair, uint64_t *idx) {
+__global__ void cn_keys(const uint32_t *src, const uint32_t *dst, uint64_t n, int undirected, int bits, uint64_t *dir) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t s = src[i], d = dst[i];
         if (undirected) {
@@ -38,6 +37,12 @@ __global__ void cn_keys(const uint32_t *src, const uint32_t *dst, uint64_t n, in
         } else {
             dir[i] = (s << bits) | d;
         }
+    }
+}
+
+__global__ void cn_pairs(const uint32_t *src, const uint32_t *dst, uint64_t n, int bits, uint64_t *pair, uint64_t *idx) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t s = src[i], d = dst[i];
         pair[i] = s < d ? (s << bits) | d : (d << bits) | s;
         idx[i] = i;
     }
@@ -71,7 +76,7 @@ constexpr int kHubLog = 7;
 
 struct CnHubs {
     uint32_t *hist;    // [33] rows by length (floor of log2 + 1); then [33]: shortest length that gets a bitmap, [34]: slots given
-    int32_t *slot;     // [v_num] bitmap of the vertex's row, -1: none
+    int32_t *slot;     // [v_num] bitmap of the vertex's row, -1: none (NULL: no row has one)
     uint32_t *bits;    // [slots][words]
     uint32_t slots, words;
 };
@@ -138,7 +143,7 @@ __global__ void cn_count(const uint64_t *pair_sorted, const uint64_t *idx_sorted
         const bool first_long = n1 > n2;                 // gcn.cpp:166-172
         const uint32_t *sh = first_long ? r2 : r1, *lg = first_long ? r1 : r2;
         const uint64_t ns = first_long ? n2 : n1, nl = first_long ? n1 : n2;
-        const int32_t slot = h.slot[first_long ? s : d];
+        const int32_t slot = h.slot ? h.slot[first_long ? s : d] : -1;
         const uint32_t *bits = h.bits + (slot < 0 ? 0 : (uint64_t)slot * h.words);
         unsigned long long count = 0, dups = 0, sd = 0;
         uint64_t first = ~0ull;
@@ -215,23 +220,34 @@ extern "C" int dg_common_neighbours(const uint32_t *src, const uint32_t *dst, ui
     const uint64_t n = n_edges, m = undirected ? 2 * n : n;
     const unsigned grid = (unsigned)dg::sm_count(device) * 8;
     // One allocation for everything (each costs hundreds of microseconds), cut into
-    // 256-byte aligned parts; the two sorts share the larger one's scratch.
+    // 256-byte aligned parts.  The rows' keys are done with when the pairs' are made, and
+    // the pairs' sort before the counts: each takes the place of the one before, so the
+    // call needs no more memory (64 bytes an edge, 60 of a directed graph, and 8 a vertex,
+    // beside the bitmaps) than one with an array each, freed in turn.  Where the bitmaps'
+    // room is refused, the call does without them.
     const int key_bits = bits_of(v_num);
     size_t cub_rows = 0, cub_pairs = 0;
     DG_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, cub_rows, (uint64_t *)nullptr, (uint64_t *)nullptr, m, 0, 2 * key_bits, s));
     DG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, cub_pairs, (uint64_t *)nullptr, (uint64_t *)nullptr,
                                             (uint64_t *)nullptr, (uint64_t *)nullptr, n, 0, 2 * key_bits, s));
-    const size_t cub_bytes = std::max(cub_rows, cub_pairs);
     size_t need = 0;
     auto part = [&](size_t bytes) {
         const size_t at = need;
         need += (bytes + 255) / 256 * 256;
         return at;
     };
-    const size_t o_src = part(n * 4), o_dst = part(n * 4), o_nbr = part(m * 4), o_off = part(((size_t)v_num + 1) * 8),
-                 o_dir = part(m * 8), o_dir2 = part(m * 8), o_pair = part(n * 8), o_pair2 = part(n * 8),
-                 o_idx = part(n * 8), o_idx2 = part(n * 8), o_sorted = part(n * 4), o_cn = part(n * 4),
-                 o_cub = part(cub_bytes ? cub_bytes : 1);
+    const size_t o_src = part(n * 4), o_dst = part(n * 4), o_nbr = part(m * 4), o_off = part(((size_t)v_num + 1) * 8);
+    const size_t o_shared = need;
+    const size_t o_dir = part(m * 8), o_dir2 = part(m * 8), o_cub_rows = part(cub_rows);
+    const size_t rows_end = need;
+    need = o_shared;
+    const size_t o_pair = part(n * 8), o_pair2 = part(n * 8), o_idx = part(n * 8), o_idx2 = part(n * 8), o_cub_pairs = need;
+    part(cub_pairs);
+    const size_t pairs_end = need;
+    need = o_cub_pairs;
+    const size_t o_sorted = part(n * 4), o_cn = part(n * 4);
+    need = std::max(need, std::max(rows_end, pairs_end));
+    const size_t plain_need = need;
     CnHubs hubs{};
     hubs.words = (v_num + 31) / 32;
     // No more rows than this can have 2^kHubLog entries.
@@ -239,39 +255,49 @@ extern "C" int dg_common_neighbours(const uint32_t *src, const uint32_t *dst, ui
     const size_t hub_bytes = (size_t)hubs.slots * hubs.words * 4;
     const size_t o_hist = part(35 * 4), o_slot = part((size_t)v_num * 4), o_bits = part(hub_bytes);
     dg::DevArray<uint8_t> block;
-    DG_CUDA(block.alloc(need));
-    uint32_t *const d_src = reinterpret_cast<uint32_t *>(block.p + o_src), *const d_dst = reinterpret_cast<uint32_t *>(block.p + o_dst),
-             *const nbr = reinterpret_cast<uint32_t *>(block.p + o_nbr);
-    uint64_t *const offsets = reinterpret_cast<uint64_t *>(block.p + o_off), *const dir = reinterpret_cast<uint64_t *>(block.p + o_dir),
-             *const dir2 = reinterpret_cast<uint64_t *>(block.p + o_dir2), *const pair = reinterpret_cast<uint64_t *>(block.p + o_pair),
-             *const pair2 = reinterpret_cast<uint64_t *>(block.p + o_pair2), *const idx = reinterpret_cast<uint64_t *>(block.p + o_idx),
-             *const idx2 = reinterpret_cast<uint64_t *>(block.p + o_idx2);
+    if (hubs.slots) {
+        const cudaError_t e = block.alloc(need);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            hubs.slots = 0;
+        } else {
+            DG_CUDA(e);
+        }
+    }
+    if (!hubs.slots) DG_CUDA(block.alloc(plain_need));
+    auto u32 = [&](size_t at) { return reinterpret_cast<uint32_t *>(block.p + at); };
+    auto u64 = [&](size_t at) { return reinterpret_cast<uint64_t *>(block.p + at); };
+    uint32_t *const d_src = u32(o_src), *const d_dst = u32(o_dst), *const nbr = u32(o_nbr);
+    uint64_t *const offsets = u64(o_off), *const dir = u64(o_dir), *const dir2 = u64(o_dir2), *const pair = u64(o_pair),
+             *const pair2 = u64(o_pair2), *const idx = u64(o_idx), *const idx2 = u64(o_idx2);
     int32_t *const cn_sorted = reinterpret_cast<int32_t *>(block.p + o_sorted), *const d_cn = reinterpret_cast<int32_t *>(block.p + o_cn);
     DG_CUDA(cudaMemcpyAsync(d_src, src, n * 4, cudaMemcpyHostToDevice, s));
     DG_CUDA(cudaMemcpyAsync(d_dst, dst, n * 4, cudaMemcpyHostToDevice, s));
-    cn_keys<<<grid, 256, 0, s>>>(d_src, d_dst, n, undirected, key_bits, dir, pair, idx);
+    cn_keys<<<grid, 256, 0, s>>>(d_src, d_dst, n, undirected, key_bits, dir);
     dg::note_launch();
     DG_CUDA(cudaGetLastError());
     // Row-sorted CSR (gcn.cpp:130-137 sorts every row by neighbour).
-    size_t bytes = cub_bytes;
-    DG_CUDA(cub::DeviceRadixSort::SortKeys(block.p + o_cub, bytes, dir, dir2, m, 0, 2 * key_bits, s));
+    DG_CUDA(cub::DeviceRadixSort::SortKeys(block.p + o_cub_rows, cub_rows, dir, dir2, m, 0, 2 * key_bits, s));
     cn_rows<<<grid, 256, 0, s>>>(dir2, m, v_num, key_bits, offsets, nbr);
     dg::note_launch();
     DG_CUDA(cudaGetLastError());
-    hubs.hist = reinterpret_cast<uint32_t *>(block.p + o_hist);
-    hubs.slot = reinterpret_cast<int32_t *>(block.p + o_slot);
-    hubs.bits = reinterpret_cast<uint32_t *>(block.p + o_bits);
-    DG_CUDA(cudaMemsetAsync(hubs.hist, 0, 35 * 4, s));
-    if (hub_bytes) DG_CUDA(cudaMemsetAsync(hubs.bits, 0, hub_bytes, s));
-    cn_lengths<<<grid, 256, 0, s>>>(offsets, v_num, hubs);
-    cn_pick<<<1, 1, 0, s>>>(hubs);
-    cn_slots<<<grid, 256, 0, s>>>(offsets, v_num, hubs);
-    cn_bits<<<grid, 256, 0, s>>>(dir2, m, key_bits, hubs);
-    dg::note_launches(4);
-    DG_CUDA(cudaGetLastError());
+    if (hubs.slots) {
+        hubs.hist = u32(o_hist);
+        hubs.slot = reinterpret_cast<int32_t *>(block.p + o_slot);
+        hubs.bits = u32(o_bits);
+        DG_CUDA(cudaMemsetAsync(hubs.hist, 0, 35 * 4, s));
+        DG_CUDA(cudaMemsetAsync(hubs.bits, 0, hub_bytes, s));
+        cn_lengths<<<grid, 256, 0, s>>>(offsets, v_num, hubs);
+        cn_pick<<<1, 1, 0, s>>>(hubs);
+        cn_slots<<<grid, 256, 0, s>>>(offsets, v_num, hubs);
+        cn_bits<<<grid, 256, 0, s>>>(dir2, m, key_bits, hubs);
+        dg::note_launches(4);
+        DG_CUDA(cudaGetLastError());
+    }
     // Pairs grouped by unordered key, input order kept inside a group (stable sort).
-    bytes = cub_bytes;
-    DG_CUDA(cub::DeviceRadixSort::SortPairs(block.p + o_cub, bytes, pair, pair2, idx, idx2, n, 0, 2 * key_bits, s));
+    cn_pairs<<<grid, 256, 0, s>>>(d_src, d_dst, n, key_bits, pair, idx);
+    dg::note_launch();
+    DG_CUDA(cub::DeviceRadixSort::SortPairs(block.p + o_cub_pairs, cub_pairs, pair, pair2, idx, idx2, n, 0, 2 * key_bits, s));
     cn_count<<<grid, 256, 0, s>>>(pair2, idx2, n, d_src, d_dst, offsets, nbr, hubs, cn_sorted);
     dg::note_launch();
     cn_scatter<<<grid, 256, 0, s>>>(pair2, idx2, n, cn_sorted, d_cn);

@@ -1,8 +1,8 @@
 // Hogwild CBOW on FP32 rows (cbow_kernel, word2vec.cu:401-509), two centres at a
 // time: the form of DG_SGNS_CBOW that trains walks of at most 32 tokens with rows
-// of up to 128 columns and up to five negatives, or, with hierarchical softmax, up
-// to 256 columns and eight negatives (sgns_cbow_kernel, dg_sgns_w2v.cu, trains the
-// others and the one-warp deterministic runs).
+// of 128 columns (sizes 65 to 128) and up to five negatives, or, with hierarchical
+// softmax, up to 256 columns and eight negatives (sgns_cbow_kernel, dg_sgns_w2v.cu,
+// trains the others and the one-warp deterministic runs).
 //
 // What bounds the rule is the L2's reduction rate.  A centre with cw contexts and
 // n negatives reads cw + 1 + n rows and adds to as many; on rows that L2 holds, a
@@ -14,32 +14,36 @@
 // of both centres' e in one atomic: 6.2 row reads and reductions a centre for the
 // contexts, not 9.
 //
-// Measured on a B200, size 128, window 10, negative 5: a YouTube-shaped round
-// (25.0M tokens) in 33.0 ms instead of 43.8; a round of the 10,000-vertex graph
-// at size 100, whose padding columns are no longer moved, in 0.38 ms instead of
-// 0.54.  What bounds it now: the same L2 reductions (12.2 rows a centre, 1.06 ns of
-// 1.32 ns a token; its reads are 0.35 ns more where the two do not overlap), then
-// DRAM (5 KB a token, 0.76 ns).
+// Measured on a B200, size 128, window 10, negative 5: two YouTube-shaped rounds with
+// their read-back in 101 ms instead of 115, three of the 10,000-vertex graph at size
+// 100 (whose padding columns are no longer moved) in 1.76 ms instead of 2.29.  What
+// bounds it now: the L2 reductions (12.2 rows a centre, 1.06 ns a token), DRAM (5 KB a
+// token, 0.76 ns), and the latency of a turn's four groups of targets.
 //
 // A Hogwild run's rows depend on how many updates are under way unseen and on how
 // many walks are trained at once.  So 16 warps of an SM train two centres each,
 // where sgns_cbow_kernel's 32 train one, and each holds two walks that it trains in
-// turn: 32 walks, 32 centres under way.  Measured against sgns_cbow_kernel's rows,
-// over the distance of two equal runs of that kernel (graphs of 10,000 to 1.1M
-// vertices, windows 1 to 10, a job's last learning rate):
+// turn: 32 walks, 32 centres under way; and the targets are read as that kernel reads
+// them, after the mean, three at a time, each group written before the next is read.
+// All of them read before the contexts were 9 % faster (92 ms), but an output row then
+// misses twice as much, and whole jobs from learning rate 0.025 ended 0.0043 lower in
+// link-prediction AUC (32 jobs on the 10,000-vertex graph; all at once after the mean:
+// 0.0012; as here: 0.0002 +- 0.0002).
+// Measured against sgns_cbow_kernel's rows, over the distance of two equal runs of that
+// kernel (graphs of 10,000 to 1.1M vertices, windows 1 to 10, a job's last learning rate):
 //   columns   negatives   input rows   output rows
-//   32..128   0..5        1.1 .. 2.4   1.0 .. 1.7
-//   32..128   7, 8        1.8 .. 2.5   1.5 .. 1.9
-//   200, 256  3..8        1.7 .. 7.2   1.3 .. 4.4    (no hierarchical softmax)
+//   65..128   0..5        1.1 .. 2.2   1.0 .. 1.7
+//   65..128   7, 8        2.1 .. 3.0   1.6 .. 2.0
+//   32, 64    1..8        1.2 .. 3.0   1.1 .. 1.8
+//   200, 256  3..8        1.9 .. 3.1   1.2 .. 2.8    (no hierarchical softmax)
 //   64..256   3..8, HS    0.9 .. 1.8   0.9 .. 1.3
-// Hence the rule: at 256 columns sgns_cbow_kernel's registers leave it eight warps, so
-// eight warps of two centres have twice as many under way; and with more negatives
-// than five single values end further off than that kernel's own runs show.  With
-// hierarchical softmax the updates of the rows near the root outweigh all that, and
-// both kernels' runs differ alike.
-// Other schedules were further off: 14 or 12 warps of 16 (up to 4.9 and 6.0), targets
-// read in groups of two to four after the contexts (up to 3.0, and 5 to 15 % slower at
-// 64 columns), four centres at a time (8.06 ms for 300,000 walks, two: 9.3).
+// Hence the rule: with more negatives than five, and at 64 columns on small graphs, single
+// values end further off than that kernel's own runs show; at 256 columns its registers
+// leave it eight warps, so eight warps of two centres have twice as many under way.  With
+// hierarchical softmax the updates of the rows near the root outweigh all that, and both
+// kernels' runs differ alike.
+// Other schedules were further off: 14 or 12 warps of 16 (up to 4.9 and 6.0), four
+// centres at a time (8.06 ms for 300,000 walks, two: 9.3).
 #include "dg_pair_grid.h"
 #include "dg_sgns.h"
 #include "dg_sgns_dev.cuh"
@@ -52,8 +56,9 @@ constexpr int kCbowWarps = 8;             // warps of a block
 constexpr uint32_t kCbowMaxTokens = 32;   // a lane per token
 constexpr int kCbowPairNeg = 5;           // the largest negative count of this kernel
 constexpr int kCbowPairHsNeg = 8;         // the same with hierarchical softmax
-constexpr int kCbowPairSize = 128;        // the largest row without it
+constexpr int kCbowPairSize = 128;        // the row without it
 
+constexpr int cbow_pair_group(int vec) { return vec <= 2 ? 4 : vec == 4 ? 3 : 2; }   // target rows read together, as sgns_cbow_kernel
 constexpr int cbow_pair_walks(int vec) { return vec <= 4 ? 2 : 1; }    // walks that a warp trains in turn
 constexpr int cbow_pair_blocks(int vec) { return vec <= 4 ? 2 : 1; }   // blocks per SM
 
@@ -100,7 +105,7 @@ struct CbowWalk {
 // warp's own updates are all seen.  Target rows are read when their centre
 // starts, after the reductions of the centre before.
 //
-// FIXED: NS negatives (5, word2vec's default), else up to NS, read from a.negative.
+// Room for NS negatives; FIXED: NS of them (word2vec's default), else a.negative.
 //
 // HS: hierarchical softmax over the centre's Huffman path before its targets
 // (word2vec.cu:436-455; hs_path, dg_sgns_dev.cuh).  Every path runs through the
@@ -112,10 +117,11 @@ struct CbowWalk {
 // each another slice's, and a path's nodes are read four at a time.
 // A round of the 50,000-vertex graph, size 128, window 5, with its read-back:
 // 11.4 -> 7.2 ms.
-template <int VEC, int NS, bool FIXED, bool HS>
+template <int VEC, bool HS, bool FIXED>
 __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
     sgns_cbow_pair_kernel(SgnsArgs a, WalkSet ws, uint32_t walks, float *hot, int32_t hot_from) {
-    constexpr int D = 32 * VEC, M = pow2_at_least(NS + 1), GROUP = 32 / M;
+    constexpr int NS = HS ? kCbowPairHsNeg : kCbowPairNeg;
+    constexpr int D = 32 * VEC, G = cbow_pair_group(VEC), M = pow2_at_least(G), GROUP = 32 / M;
     constexpr int BATCH = VEC <= 4 ? 8 : 4;   // context rows in flight together
     constexpr uint32_t kAll = 0xffffffffu;
     __shared__ __align__(16) int32_t sen_all[kCbowWarps][2][kCbowMaxTokens];
@@ -184,19 +190,6 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
             return;
         }
     };
-    // The target rows of centre p (a target that does not train reads the centre's row, unused).
-    struct Targets {
-        int32_t t[NS + 1];
-        RowVec<VEC> row[NS + 1];
-    };
-    auto load_targets = [&](uint32_t p, Targets &q) {
-        q.t[0] = A.sen[p];
-#pragma unroll
-        for (int j = 0; j < NS; j++) q.t[j + 1] = j < neg ? A.negs[p * NS + j] : q.t[0];
-#pragma unroll
-        for (int j = 0; j <= NS; j++)
-            if (j <= neg) load_row<VEC>(out_row(q.t[j]), q.row[j]);
-    };
     // The target rows of centre p of walk W on their way to L2, a lane per row.
     auto prefetch_targets = [&](const CbowWalk &W, uint32_t p) {
         if (p >= W.n || (int)lane > neg) return;
@@ -204,36 +197,49 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
         prefetch_l2(a.syn1 + (size_t)t * D, D * 4);
     };
     // Centre p's targets against x, the mean of its context rows: e receives the
-    // gradient of x, the target rows their updates (word2vec.cu:453-497).
-    auto train_targets = [&](uint32_t p, const RowVec<VEC> &x, RowVec<VEC> &e, Targets &q) {
+    // gradient of x, the target rows their updates (word2vec.cu:453-497).  G rows are
+    // read together, after the mean, and their updates sent before the next are read.
+    auto train_targets = [&](uint32_t p, const RowVec<VEC> &x, RowVec<VEC> &e) {
         const uint32_t fl = __shfl_sync(kAll, A.flags, p);
-        if (!(fl & 0x80000000u)) {   // all sums and gradients at once
-            float f[M];
 #pragma unroll
-            for (int j = 0; j < M; j++) f[j] = j <= NS && j <= neg && own ? row_dot(x, q.row[j <= NS ? j : 0]) : 0.f;
-            const float mine = warp_sums_split<M>(f, lane);
-            const uint32_t jm = lane / GROUP;
-            const float gm = (fl >> jm) & 1u ? sg_grad(mine, jm == 0, a.exp_table, a.alpha) : 0.f;
+        for (int g0 = 0; g0 <= NS; g0 += G) {
+            if (g0 > neg) break;
+            int32_t t[G];   // -1: no target, or one that does not train
+            RowVec<VEC> row[G];
 #pragma unroll
-            for (int j = 0; j <= NS; j++) {
-                const float g = __shfl_sync(kAll, gm, j * GROUP);
-                if (!((fl >> j) & 1u)) continue;
-                row_fma(e, g, q.row[j]);
-                if (own) add_row<VEC>(out_row(q.t[j]), row_mul(g, x));
+            for (int k = 0; k < G; k++) {
+                const int j = g0 + k;
+                t[k] = j == 0 ? A.sen[p] : j <= NS && ((fl >> j) & 1u) ? A.negs[p * NS + j - 1] : -1;
+                if (t[k] >= 0) load_row<VEC>(out_row(t[k]), row[k]);
+                else zero_row(row[k]);
             }
-        } else {   // a target repeats: one after the other, each seeing the updates before it
+            if (!(fl & 0x80000000u)) {   // the group's sums and gradients at once
+                float f[M];
 #pragma unroll
-            for (int j = 0; j <= NS; j++) {
-                if (!((fl >> j) & 1u)) continue;
-                if (!own) zero_row(q.row[j]);
-                const float g = sg_grad(warp_dot<VEC>(x, q.row[j]), j == 0, a.exp_table, a.alpha);
-                row_fma(e, g, q.row[j]);
-                const RowVec<VEC> upd = row_mul(g, x);
-                row_add(q.row[j], upd);
-                if (own) add_row<VEC>(out_row(q.t[j]), upd);
+                for (int k = 0; k < M; k++) f[k] = k < G && own ? row_dot(x, row[k < G ? k : 0]) : 0.f;
+                const float mine = warp_sums_split<M>(f, lane);
+                const float gm = sg_grad(mine, g0 == 0 && lane < GROUP, a.exp_table, a.alpha);
 #pragma unroll
-                for (int k = j + 1; k <= NS; k++)
-                    if (q.t[k] == q.t[j]) q.row[k] = q.row[j];
+                for (int k = 0; k < G; k++) {
+                    const float g = __shfl_sync(kAll, gm, k * GROUP);
+                    if (t[k] < 0) continue;
+                    row_fma(e, g, row[k]);
+                    if (own) add_row<VEC>(out_row(t[k]), row_mul(g, x));
+                }
+            } else {   // a target repeats: one after the other, each seeing the updates before it
+#pragma unroll
+                for (int k = 0; k < G; k++) {
+                    if (t[k] < 0) continue;
+                    if (!own) zero_row(row[k]);
+                    const float g = sg_grad(warp_dot<VEC>(x, row[k]), g0 + k == 0, a.exp_table, a.alpha);
+                    row_fma(e, g, row[k]);
+                    const RowVec<VEC> upd = row_mul(g, x);
+                    row_add(row[k], upd);
+                    if (own) add_row<VEC>(out_row(t[k]), upd);
+#pragma unroll
+                    for (int q = k + 1; q < G; q++)
+                        if (t[q] == t[k]) row[q] = row[k];
+                }
             }
         }
     };
@@ -298,10 +304,9 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
             const uint32_t wp = __shfl_sync(kAll, A.win, p);
             const uint32_t wq = p + 1 < A.n ? __shfl_sync(kAll, A.win, (p + 1) & 31) : 0u;
             const uint32_t all = wp | wq, b0 = ((uint32_t)__ffs(all) - 1) & ~3u;
+            if (walks == 1) prefetch_targets(A, p);
             prefetch_targets(A, p + 1);
             prefetch_targets(B, B.p);
-            Targets q;
-            if (!HS) load_targets(p, q);
             // Context rows of both centres, summed in window order (word2vec.cu:419-428).
             RowVec<VEC> x, y, e;
             zero_row(x);
@@ -326,22 +331,15 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
             }
             mean(x, wp);
             zero_row(e);
-            if (HS) {
-                train_path(p, x, e);
-                load_targets(p, q);
-            }
-            train_targets(p, x, e, q);
+            if (HS) train_path(p, x, e);
+            train_targets(p, x, e);
             if (wq) {
-                if (!HS) load_targets(p + 1, q);
                 const int pairs = __reduce_add_sync(kAll, ((wq >> lane) & 1u) ? __popc(A.same & wp) : 0);
                 if (pairs) row_fma(y, (float)pairs, e);   // 0 of an infinite e would be no number
                 mean(y, wq);
                 zero_row(x);   // from here the second centre's e
-                if (HS) {
-                    train_path(p + 1, y, x);
-                    load_targets(p + 1, q);
-                }
-                train_targets(p + 1, y, x, q);
+                if (HS) train_path(p + 1, y, x);
+                train_targets(p + 1, y, x);
             }
             // e to every context row (word2vec.cu:498-505), both centres' at once.
             for (uint32_t b = b0; b < 32 && (all >> b); b += 4) {
@@ -376,13 +374,13 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
 
 bool cbow_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
     return s->p.mode == DG_SGNS_CBOW && !s->p.deterministic && ws.max_len > 0 && ws.max_len <= kCbowMaxTokens &&
-           s->p.size <= (a.hs ? 256 : kCbowPairSize) && a.negative <= (a.hs ? kCbowPairHsNeg : kCbowPairNeg) &&
+           (a.hs ? s->p.size <= 256 : s->p.size == kCbowPairSize) && a.negative <= (a.hs ? kCbowPairHsNeg : kCbowPairNeg) &&
            a.vocab_size > 1;
 }
 
-template <int V, int NS, bool FIXED, bool HS>
+template <int V, bool HS, bool FIXED>
 static int cbow_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    auto kern = sgns_cbow_pair_kernel<V, NS, FIXED, HS>;
+    auto kern = sgns_cbow_pair_kernel<V, HS, FIXED>;
     int per_sm = 0;
     DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kCbowWarps, 0));
     const PairGrid g = pair_grid(s->p.workers, {std::min(std::max(per_sm, 1), cbow_pair_blocks(V)) * dg::sm_count(s->device),
@@ -405,17 +403,12 @@ static int cbow_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
     return DG_OK;
 }
 
-template <int V, bool HS>
-static int cbow_pair_negatives(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    if (HS && a.negative > kCbowPairNeg) return cbow_pair_launch<V, HS ? kCbowPairHsNeg : kCbowPairNeg, false, HS>(s, a, ws);
-    return a.negative == kCbowPairNeg ? cbow_pair_launch<V, kCbowPairNeg, true, HS>(s, a, ws)
-                                      : cbow_pair_launch<V, kCbowPairNeg, false, HS>(s, a, ws);
-}
-
 template <int V>
 static int cbow_pair_size(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    if (a.hs) return cbow_pair_negatives<V, true>(s, a, ws);
-    if constexpr (32 * V <= kCbowPairSize) return cbow_pair_negatives<V, false>(s, a, ws);
+    if (a.hs) return cbow_pair_launch<V, true, false>(s, a, ws);
+    if constexpr (32 * V == kCbowPairSize)
+        return a.negative == kCbowPairNeg ? cbow_pair_launch<V, false, true>(s, a, ws)
+                                          : cbow_pair_launch<V, false, false>(s, a, ws);
     return dg::fail(DG_ERR_STATE, "rows of %d columns are not trained two centres at a time", 32 * V);
 }
 

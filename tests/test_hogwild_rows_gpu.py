@@ -62,7 +62,7 @@ def test_shared_negatives(corpus, size, window, negative, most):
 
 
 @pytest.mark.parametrize("size,window,negative,hs,most", [
-    (32, 6, 5, False, 4), (64, 10, 3, False, 4), (100, 8, 5, False, 4), (128, 5, 1, False, 4), (128, 9, 5, True, 4),
+    (32, 6, 5, False, 1.5), (64, 10, 5, False, 1.5), (100, 8, 5, False, 4), (128, 5, 1, False, 4), (128, 9, 5, True, 4),
     (64, 8, 8, True, 4), (256, 7, 3, True, 4), (200, 9, 5, False, 1.5), (256, 5, 5, False, 1.5), (64, 9, 8, False, 1.5),
     (128, 10, 7, False, 1.5)])
 def test_cbow(corpus, size, window, negative, hs, most):

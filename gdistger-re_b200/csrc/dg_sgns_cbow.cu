@@ -114,9 +114,13 @@ struct CbowWalk {
 // root and its two neighbours cost 1.1M tokens 9 ms of 10.3.  So for the launch the
 // kHotNodes most visited nodes' rows (the last inner nodes made, so the highest ids)
 // move to a buffer whose rows lie in eight pieces a kilobyte apart (hot_offset),
-// each another slice's, and a path's nodes are read four at a time.
-// A round of the 50,000-vertex graph, size 128, window 5, with its read-back:
-// 11.4 -> 7.2 ms.
+// each another slice's.  A path's nodes are read two at a time: a round of the
+// 50,000-vertex graph, size 128, window 5, with its read-back 11.3 -> 7.3 ms (one at a
+// time 7.4, four 7.2).  Read together, a node misses the updates that reach it while the
+// others are summed, and every centre trains the root: link-prediction AUC of whole jobs
+// on the 10,000-vertex graph (16 each) from learning rate 0.01 0.548 with hs_path, whose
+// nodes wait for one another, 0.524 with four, 0.557 with two, 0.595 with one (from
+// 0.025 0.486, 0.479, 0.483, 0.487): two is what differs least.
 template <int VEC, bool HS, bool FIXED>
 __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
     sgns_cbow_pair_kernel(SgnsArgs a, WalkSet ws, uint32_t walks, float *hot, int32_t hot_from) {
@@ -254,10 +258,10 @@ __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
         }
     };
 
-    // Centre p's path against x: the nodes are distinct, so four are read, summed and
+    // Centre p's path against x: the nodes are distinct, so two are read, summed and
     // updated together.
     auto train_path = [&](uint32_t p, const RowVec<VEC> &x, RowVec<VEC> &e) {
-        constexpr int H = 4;
+        constexpr int H = 2;
         const int32_t word = A.sen[p], k1 = a.hs_off[word + 1];
         for (int32_t k = a.hs_off[word]; k < k1; k += H) {
             int32_t point = -1;

@@ -1,10 +1,15 @@
-"""A whole CBOW job from the learning rate that jobs start with (0.025), trained by the kernel of two
+"""A whole CBOW job from a learning rate that jobs start with (0.025), trained by the kernel of two
 centres at a time and by the one-centre kernel (brought in as in test_hogwild_rows_gpu.py): the
 link-prediction AUC of the two.
 
 Seed by seed the difference varies by 0.0013 (standard deviation of 32 jobs), so the mean
 over 10 seeds by 0.0004; the bound, 0.002, is five times that.  A kernel that reads all its
-targets before the contexts, and so holds them longer unseen, loses 0.0043."""
+targets before the contexts, and so holds them longer unseen, loses 0.0043.
+
+With hierarchical softmax, from 0.01 (at 0.025 these jobs end below chance): every centre
+trains the root, so a job depends on how long a node is held, 0.047 above the one-centre
+kernel's 0.548 with one node at a time, 0.009 with two, 0.025 below with four.  The mean
+over 10 seeds varies by 0.001; the bound is 0.015."""
 import numpy as np
 import pytest
 
@@ -13,7 +18,8 @@ from distger.sgns import SGNS
 pytestmark = pytest.mark.gpu
 
 
-def test_auc_of_a_job(distger_lib):
+@pytest.mark.parametrize("hs,alpha,most", [(False, 0.025, 0.002), (True, 0.01, 0.015)])
+def test_auc_of_a_job(distger_lib, hs, alpha, most):
     from distger import WalkEngine, graphgen, lp
     from distger.embed import make_lr
     cfg = graphgen.CONFIGS["c1_small"]
@@ -24,16 +30,16 @@ def test_auc_of_a_job(distger_lib):
         eng = WalkEngine(seed=seed)
         eng.load_graph(v, "", make_undirected=True, edges=train)
         counts = np.append(np.add(*eng.graph.degrees()), 0).astype(np.uint32)
-        made = [SGNS(v + 1, counts, size=128, window=10, negative=5, sample=1e-3, alpha=0.025, min_count=1, mode="cbow",
-                     seed=seed) for _ in range(2)]
-        rate = make_lr("exp", 0.025, 30)
+        made = [SGNS(v + 1, counts, size=128, window=10, negative=5, sample=1e-3, alpha=alpha, min_count=1, mode="cbow",
+                     seed=seed, hs=hs) for _ in range(2)]
+        rate = make_lr("exp", alpha, 30)
         for r in range(1, 31):
             paths = eng.run_round(v, r)
             offs, verts = paths.to_numpy()
             paths.close()
-            alpha = rate.get_lr()
+            now = rate.get_lr()
             for s, extra in zip(made, (2, 70)):
-                s.train_host(np.append(offs, offs[-1] + extra), np.append(verts, np.full(extra, v, np.uint32)), alpha)
+                s.train_host(np.append(offs, offs[-1] + extra), np.append(verts, np.full(extra, v, np.uint32)), now)
         auc = []
         for s in made:
             rows, ids = s.embedding()
@@ -43,4 +49,4 @@ def test_auc_of_a_job(distger_lib):
             s.close()
         off.append(auc[0] - auc[1])
     print("AUC, two centres less one:", np.round(off, 4))
-    assert abs(np.mean(off)) < 0.002
+    assert abs(np.mean(off)) < most

@@ -102,8 +102,8 @@ struct CbowWalk {
 // The second centre's context rows were read before the first centre's e: they
 // are short of it by e times the number of (position of one window, position of
 // the other) pairs that hold one word, which is added to their sum.  So this
-// warp's own updates are all seen.  Target rows are read when their centre
-// starts, after the reductions of the centre before.
+// warp's own updates are all seen.  Target rows are read after their centre's
+// mean, and so after the reductions of the centre before.
 //
 // Room for NS negatives; FIXED: NS of them (word2vec's default), else a.negative.
 //
@@ -115,12 +115,14 @@ struct CbowWalk {
 // kHotNodes most visited nodes' rows (the last inner nodes made, so the highest ids)
 // move to a buffer whose rows lie in eight pieces a kilobyte apart (hot_offset),
 // each another slice's.  A path's nodes are read two at a time: a round of the
-// 50,000-vertex graph, size 128, window 5, with its read-back 11.3 -> 7.3 ms (one at a
+// 50,000-vertex graph, size 128, window 5, with its read-back 11.3 -> 7.4 ms (one at a
 // time 7.4, four 7.2).  Read together, a node misses the updates that reach it while the
 // others are summed, and every centre trains the root: link-prediction AUC of whole jobs
-// on the 10,000-vertex graph (16 each) from learning rate 0.01 0.548 with hs_path, whose
+// on the 10,000-vertex graph (16 each) from learning rate 0.01 is 0.548 with hs_path, whose
 // nodes wait for one another, 0.524 with four, 0.557 with two, 0.595 with one (from
-// 0.025 0.486, 0.479, 0.483, 0.487): two is what differs least.
+// 0.025 0.486, 0.479, 0.483, 0.487): two is what differs least.  (On the YouTube-shaped
+// graph from 0.01: 0.570 with hs_path, 0.606 here; without hierarchical softmax 0.828 in
+// both kernels.)
 template <int VEC, bool HS, bool FIXED>
 __global__ void __launch_bounds__(kCbowWarps * 32, cbow_pair_blocks(VEC))
     sgns_cbow_pair_kernel(SgnsArgs a, WalkSet ws, uint32_t walks, float *hot, int32_t hot_from) {

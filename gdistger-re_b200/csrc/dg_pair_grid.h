@@ -1,5 +1,5 @@
-// Launch shape of the kernels that train one or two walks to a warp (dg_sgns_cbow.cu,
-// dg_sgns_negshare.cu).  Host code without CUDA types.
+// Launch shape of a kernel that trains one or two walks to a warp (dg_sgns_negshare.cu).
+// Host code without CUDA types.
 #pragma once
 
 #include <algorithm>

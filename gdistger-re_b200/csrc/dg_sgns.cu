@@ -1443,7 +1443,7 @@ dg_sgns::~dg_sgns() {
         dg::DeviceGuard guard(device);
         cudaStreamSynchronize(stream);
         v2w.release(); keep_thr.release(); table.release(); exp_table.release();
-        hs_off.release(); hs_point.release(); hs_code.release(); hs_hot.release();
+        hs_off.release(); hs_point.release(); hs_code.release();
         syn0.release(); syn1.release(); in_bf.release(); out_bf.release(); in_master.release(); out_master.release();
         scratch.release(); queue.release(); stats.release(); adj_in.release(); adj_out.release(); adj_flag.release();
         adj_offs.release(); adj_pin.release(); adj_pout.release(); adj_neg.release(); adj_step.release();

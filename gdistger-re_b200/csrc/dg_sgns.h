@@ -124,9 +124,6 @@ bool bf_staging_safe(const std::vector<uint32_t> &cn, uint32_t n_master, int neg
 int launch_minibatch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
 // cbow_kernel and __sgNegReuse semantics (dg_sgns_w2v.cu).
 int launch_cbow(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
-// The Hogwild form of CBOW that trains two centres at a time (dg_sgns_cbow.cu) and what it takes.
-bool cbow_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
-int launch_cbow_pair(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
 int launch_plain_hs(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws);
 // word2vec's Huffman coding (CreateBinaryTree, word2vec.cu:684-740) of counts in
 // vocabulary order, laid out as off[n + 1] / point / code.  false if a code
@@ -212,7 +209,6 @@ struct dg_sgns {
     uint64_t adj_exec_k = 0;
     dg::DevArray<int32_t> hs_off, hs_point;   // hierarchical softmax: Huffman paths (dgs::huffman_codes)
     dg::DevArray<int8_t> hs_code;
-    dg::DevArray<float> hs_hot;               // CBOW: rows of the nodes near the root during a launch (dg_sgns_cbow.cu)
     dg::DevArray<uint32_t> queue;
     dg::DevArray<unsigned long long> stats;
     dg::DevArray<uint64_t> host_off;     // dg_sgns_train_host: device copies of the caller's walks,

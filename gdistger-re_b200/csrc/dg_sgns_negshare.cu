@@ -13,7 +13,7 @@
 // rows of 256) are not moved.
 //
 // A Hogwild run's rows depend on how many pairs are under way unseen and on how
-// many walks are trained at once (dg_sgns_cbow.cu), so half as many warps as
+// many walks are trained at once, so half as many warps as
 // sgns_negshare_kernel's hold two walks each and train two pairs of either in turn.
 //
 // A round of the 50,000-vertex graph at size 200, window 5, negative 5, with its

@@ -421,7 +421,6 @@ static int negshare_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
 }
 
 int launch_cbow(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    if (cbow_pair_applies(s, a, ws)) return launch_cbow_pair(s, a, ws);
     if (s->p.mode == DG_SGNS_CBOW_BF16) {
         switch (s->p.size / 32) {
             case 2: return cbow_launch<2, true>(s, a, ws);

@@ -170,9 +170,9 @@ typedef struct {
     uint64_t table_size; /* unigram table slots; 0 = 1e8 (word2vec.cu:66) */
     uint32_t master_rows; /* minibatch mode: hottest rows kept in FP32; 0 = 65536, >= vocabulary = all */
     uint32_t workers;     /* concurrent trainer workers: walks under way (a warp each, or two walks to a warp
-                             in DG_SGNS_CBOW and DG_SGNS_SG_SHARED where the count asks for it), CTAs in
-                             minibatch mode; from a block's warps on rounded up to whole blocks; 0 =
-                             automatic; capped at what the GPU holds resident.  Adjoint mode:
+                             in DG_SGNS_SG_SHARED where the count asks for it), CTAs in minibatch mode; from
+                             a block's warps on rounded up to whole blocks; 0 = automatic; capped at what
+                             the GPU holds resident.  Adjoint mode:
                              minibatches per gradient step (0 = automatic bound) */
     int hs;               /* -hs 1: hierarchical softmax over word2vec's Huffman coding of the vocabulary
                              (CreateBinaryTree, word2vec.cu:684-740) before the negative-sampling

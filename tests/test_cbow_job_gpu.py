@@ -1,15 +1,14 @@
-"""A whole CBOW job from a learning rate that jobs start with (0.025), trained by the kernel of two
-centres at a time and by the one-centre kernel (brought in as in test_hogwild_rows_gpu.py): the
+"""A whole CBOW job from a learning rate that jobs start with (0.025), trained by the kernel that
+a call takes and by the one-centre kernel (brought in as in test_hogwild_rows_gpu.py): the
 link-prediction AUC of the two.
 
 Seed by seed the difference varies by 0.0013 (standard deviation of 32 jobs), so the mean
-over 10 seeds by 0.0004; the bound, 0.002, is five times that.  A kernel that reads all its
-targets before the contexts, and so holds them longer unseen, loses 0.0043.
-
-With hierarchical softmax, from 0.01 (at 0.025 these jobs end below chance): every centre
-trains the root, so a job depends on how long a node is held, 0.047 above the one-centre
-kernel's 0.548 with one node at a time, 0.009 with two, 0.025 below with four.  The mean
-over 10 seeds varies by 0.001; the bound is 0.015."""
+over 10 seeds by 0.0004; the bound, 0.002, is five times that.  (A kernel of two centres at a
+time whose targets were read before the contexts, and so held longer unseen, lost 0.0043.)
+With hierarchical softmax, from 0.01 (at 0.025 these jobs end below chance), every centre
+trains the root, and a job depends on how long a node is held: four nodes of a path read
+together lost 0.025, one at a time from spread rows gained 0.047.  The mean over 10 seeds
+varies by 0.001; the bound is 0.015."""
 import numpy as np
 import pytest
 
@@ -48,5 +47,5 @@ def test_auc_of_a_job(distger_lib, hs, alpha, most):
             auc.append(lp.evaluate(by_vertex[:v], pairs, labels)["auc"])
             s.close()
         off.append(auc[0] - auc[1])
-    print("AUC, two centres less one:", np.round(off, 4))
+    print("AUC, difference:", np.round(off, 4))
     assert abs(np.mean(off)) < most

@@ -1,5 +1,5 @@
-"""The CBOW pair kernel (dg_sgns_cbow.cu) run by one warp, measured against what a run
-changes, and both pair kernels with two walks to a warp.
+"""Hogwild CBOW run by one warp, measured against what a run changes, and the shared-negative
+pair kernel with two walks to a warp.
 
 One warp: as test_negshare_updates_gpu.py, the difference from the sequential run relative
 to the update, on walks that step back (the windows of neighbouring centres then hold one
@@ -8,7 +8,7 @@ of some 960 terms by 0.003 / 0.5, 1.9e-4 of the update at most; the bound, 4e-4,
 two.  With hierarchical softmax the change also moves the root's row, which enters every
 later centre: a NumPy model of the rule shows up to 4.0e-4 for one crossing in 120 runs
 (5e-7 without); the bound there is 2e-3.  In that model the rows are 1.3e-2 off (7.9e-2 with
-hierarchical softmax) where the second centre's mean misses the first one's update.
+hierarchical softmax) where one centre's mean misses the update of the centre before.
 
 Two walks: more walks than warps, each of words that no other walk holds, so that only the
 negatives' rows are shared; at this learning rate runs whose walks see none or all of each

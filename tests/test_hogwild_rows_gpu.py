@@ -1,15 +1,15 @@
-"""Hogwild rows of the kernels that train two pairs (centres) at a time, against the kernels
-that train one.
+"""Hogwild rows of the kernel that a call takes, against those of the kernels that train one pair
+(centre) at a time.
 
 A Hogwild run depends on which updates see each other, so a kernel that trains faster
 also trains a little differently.  Measured here: how far the rows of the kernel that a
 call takes end from those of the one-at-a-time kernel, over how far two equal runs of
 that kernel end from each other (the median of six pairs of runs).  Where the call takes
 the one-at-a-time kernel itself this is 1 but for chance (medians of 0.9 to 1.1): at most
-1.5.  Where it takes the pair kernel, at most 4.
+1.5.  Where it takes the shared-negative pair kernel, at most 4.
 
 The one-at-a-time kernel is reached with the same tokens: one more walk, longer than the
-pair kernels take, of a vertex that is not in the vocabulary.  Rows and learning rate are
+pair kernel takes, of a vertex that is not in the vocabulary.  Rows and learning rate are
 those of a job's last rounds."""
 import itertools
 
@@ -61,9 +61,8 @@ def test_shared_negatives(corpus, size, window, negative, most):
     assert max(_ratios(corpus, mode="sg_shared", size=size, window=window, negative=negative)) <= most
 
 
-@pytest.mark.parametrize("size,window,negative,hs,most", [
-    (32, 6, 5, False, 1.5), (64, 10, 5, False, 1.5), (100, 8, 5, False, 4), (128, 5, 1, False, 4), (128, 9, 5, True, 4),
-    (64, 8, 8, True, 4), (256, 7, 3, True, 4), (200, 9, 5, False, 1.5), (256, 5, 5, False, 1.5), (64, 9, 8, False, 1.5),
-    (128, 10, 7, False, 1.5)])
-def test_cbow(corpus, size, window, negative, hs, most):
-    assert max(_ratios(corpus, mode="cbow", size=size, window=window, negative=negative, hs=hs)) <= most
+@pytest.mark.parametrize("size,window,negative,hs", [
+    (32, 6, 5, False), (64, 10, 5, False), (100, 8, 5, False), (128, 5, 1, False), (128, 9, 5, True), (64, 8, 8, True),
+    (256, 7, 3, True), (200, 9, 5, False), (256, 5, 5, False), (64, 9, 8, False), (128, 10, 7, False)])
+def test_cbow(corpus, size, window, negative, hs):
+    assert max(_ratios(corpus, mode="cbow", size=size, window=window, negative=negative, hs=hs)) <= 1.5

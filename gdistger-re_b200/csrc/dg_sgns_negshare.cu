@@ -1,6 +1,6 @@
 // Hogwild shared-negative skip-gram on FP32 rows (__sgNegReuse, word2vec.cu:231-303),
 // two pairs at a time: the form of DG_SGNS_SG_SHARED that trains walks of at most
-// 64 tokens with rows of 64 to 256 columns and three to five negatives
+// 64 tokens with rows of 256 columns (sizes 129 to 256) and four or five negatives
 // (sgns_negshare_kernel, dg_sgns_w2v.cu, trains the others and the deterministic
 // runs).
 //
@@ -13,38 +13,35 @@
 // rows of 256) are not moved.
 //
 // A Hogwild run's rows depend on how many pairs are under way unseen and on how
-// many walks are trained at once, so half as many warps as
-// sgns_negshare_kernel's hold two walks each and train two pairs of either in turn.
+// many walks are trained at once, so half as many warps as sgns_negshare_kernel's
+// hold two walks each and train two pairs of either in turn.
 //
 // A round of the 50,000-vertex graph at size 200, window 5, negative 5, with its
-// read-back: 21.2 -> 12.1 ms.
+// read-back: 21.3 -> 11.9 ms.
 //
-// Why three to five negatives.  Each negative row is read once for two pairs, so it
-// misses the updates of about twice as many pairs of other walks, and its share of a
-// walk's updates grows with their number: on graphs of 10,000 to 200,000 vertices, sizes
-// 64 to 256, the rows end 1.0 to 1.6 times as far (2.0 at 200 columns and three
-// negatives, once) from the one-pair kernel's as two equal runs of that kernel from each
-// other with three to five negatives, but up to 3.0 times with seven and 2.5 with eight
-// (64 columns the worst; single values leave what that kernel's own runs show).  Below
-// three there is too little to share: 40,000 vertices, size 64, window 8 takes 3.9 ms
-// against 3.3 with one negative, 120,000 at size 128, window 5 10.6 against 10.7 with
-// two, while three (40,000, size 64, window 10) take 4.8 against 5.4 and four (200,000,
-// size 100, window 6) 20.6 against 26.8.
+// Why 256 columns and four or five negatives.  Each negative row is read once for two
+// pairs, so it misses the updates of more pairs of other walks.  Over the distance of two
+// equal runs of the one-pair kernel from each other (graphs of 10,000 to 200,000
+// vertices), rows of 256 columns with four or five negatives end 0.9 to 1.6 times as far
+// from that kernel's after one pass and 1.0 to 2.5 times after two (its own runs: 1.5 to
+// 2.2).  With three they are up to 2.0 and 2.7 times as far, with seven and eight up to
+// 1.9.  At 64 and 128 columns, where that kernel has 32 warps an SM and not 16, it is up to
+// 3.0 (64 columns, seven negatives), and single values of the output rows end up to 11
+// times further off than its own runs show, on graphs of 10,000 to 16,000 vertices above
+// all.  Below three there is little to share: one negative takes 3.9 ms against 3.3
+// (40,000 vertices, size 64), two 10.6 against 10.7 (120,000, size 128).
 #include "dg_pair_grid.h"
 #include "dg_sgns.h"
 #include "dg_sgns_dev.cuh"
-
-#include <algorithm>
 
 namespace dgs {
 
 constexpr int kShareWarps = 8;             // warps of a block
 constexpr uint32_t kShareTokens = 64;      // the longest walk of this kernel
-constexpr int kShareLeastNeg = 3;          // the negative counts of this kernel
+constexpr int kShareLeastNeg = 4;          // the negative counts of this kernel
 constexpr int kShareMostNeg = 5;
-
-// Blocks per SM: two walks a warp, 32 walks up to 128 columns, 16 at 256.
-constexpr int share_pair_blocks(int vec) { return vec <= 4 ? 2 : 1; }
+constexpr int kShareSize = 256;            // the row of this kernel, kShareVec columns to a lane
+constexpr int kShareVec = kShareSize / 32;
 
 // A walk under way: its length, centre and the centre's next pair, its words and
 // negatives (shared), whether a negative occurs twice, and this lane's columns of
@@ -56,34 +53,25 @@ struct ShareWalk {
     bool repeat = false;
 };
 
-template <int VEC>
-__device__ __forceinline__ void share_put(float *p, const RowVec<VEC> &r) {
+__device__ __forceinline__ void share_put(float *p, const RowVec<kShareVec> &r) {
 #pragma unroll
-    for (int i = 0; i < VEC; i += VEC >= 4 ? 4 : 2) {
-        if constexpr (VEC >= 4) *reinterpret_cast<float4 *>(p + i) = make_float4(r.v[i], r.v[i + 1], r.v[i + 2], r.v[i + 3]);
-        else *reinterpret_cast<float2 *>(p + i) = make_float2(r.v[i], r.v[i + 1]);
-    }
+    for (int i = 0; i < kShareVec; i += 4)
+        *reinterpret_cast<float4 *>(p + i) = make_float4(r.v[i], r.v[i + 1], r.v[i + 2], r.v[i + 3]);
 }
-template <int VEC>
-__device__ __forceinline__ void share_get(const float *p, RowVec<VEC> &r) {
+__device__ __forceinline__ void share_get(const float *p, RowVec<kShareVec> &r) {
 #pragma unroll
-    for (int i = 0; i < VEC; i += VEC >= 4 ? 4 : 2) {
-        if constexpr (VEC >= 4) {
-            const float4 q = *reinterpret_cast<const float4 *>(p + i);
-            r.v[i] = q.x; r.v[i + 1] = q.y; r.v[i + 2] = q.z; r.v[i + 3] = q.w;
-        } else {
-            const float2 q = *reinterpret_cast<const float2 *>(p + i);
-            r.v[i] = q.x; r.v[i + 1] = q.y;
-        }
+    for (int i = 0; i < kShareVec; i += 4) {
+        const float4 q = *reinterpret_cast<const float4 *>(p + i);
+        r.v[i] = q.x; r.v[i + 1] = q.y; r.v[i + 2] = q.z; r.v[i + 3] = q.w;
     }
 }
 
 // Lane l owns columns [l * VEC, l * VEC + VEC) of every row.  FIXED: NS negatives
-// (word2vec's default), else up to NS, read from a.negative.
-template <int VEC, int NS, bool FIXED>
-__global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
+// (word2vec's default), else up to NS, read from a.negative.  One block to an SM.
+template <bool FIXED>
+__global__ void __launch_bounds__(kShareWarps * 32, 1)
     sgns_negshare_pair_kernel(SgnsArgs a, WalkSet ws, uint32_t walks) {
-    constexpr int D = 32 * VEC, M = pow2_at_least(NS + 1), GROUP = 32 / M;
+    constexpr int VEC = kShareVec, NS = kShareMostNeg, D = kShareSize, M = pow2_at_least(NS + 1), GROUP = 32 / M;
     constexpr uint32_t kAll = 0xffffffffu;
     __shared__ int32_t sen_all[kShareWarps][2][kShareTokens];
     __shared__ int32_t negs_all[kShareWarps][2][NS];
@@ -274,37 +262,24 @@ __global__ void __launch_bounds__(kShareWarps * 32, share_pair_blocks(VEC))
 }
 
 bool negshare_pair_applies(const dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    return !s->p.deterministic && ws.max_len > 0 && ws.max_len <= kShareTokens && s->p.size >= 64 && s->p.size <= 256 &&
+    return !s->p.deterministic && ws.max_len > 0 && ws.max_len <= kShareTokens && s->p.size == kShareSize &&
            a.negative >= kShareLeastNeg && a.negative <= kShareMostNeg && a.vocab_size > 1;
 }
 
-template <int V, int NS, bool FIXED>
+template <bool FIXED>
 static int negshare_pair_launch(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    auto kern = sgns_negshare_pair_kernel<V, NS, FIXED>;
-    int per_sm = 0;
-    const size_t smem = (size_t)kShareWarps * 4 * 32 * V * sizeof(float);
+    auto kern = sgns_negshare_pair_kernel<FIXED>;
+    const size_t smem = (size_t)kShareWarps * 4 * kShareSize * sizeof(float);
     DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kShareWarps, smem));
-    const PairGrid g = pair_grid(s->p.workers, {std::min(std::max(per_sm, 1), share_pair_blocks(V)) * dg::sm_count(s->device),
-                                                kShareWarps, 2});
+    const PairGrid g = pair_grid(s->p.workers, {dg::sm_count(s->device), kShareWarps, 2});
     kern<<<g.blocks, 32 * g.warps, smem / kShareWarps * g.warps, s->stream>>>(a, ws, g.walks);
     dg::note_launch();
     DG_CUDA(cudaGetLastError());
     return DG_OK;
 }
 
-template <int V>
-static int negshare_pair_size(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    return a.negative == kShareMostNeg ? negshare_pair_launch<V, kShareMostNeg, true>(s, a, ws)
-                                       : negshare_pair_launch<V, kShareMostNeg, false>(s, a, ws);
-}
-
 int launch_negshare_pair(dg_sgns *s, const SgnsArgs &a, const WalkSet &ws) {
-    switch (s->p.size / 32) {
-    case 2: return negshare_pair_size<2>(s, a, ws);
-    case 4: return negshare_pair_size<4>(s, a, ws);
-    default: return negshare_pair_size<8>(s, a, ws);
-    }
+    return a.negative == kShareMostNeg ? negshare_pair_launch<true>(s, a, ws) : negshare_pair_launch<false>(s, a, ws);
 }
 
 }  // namespace dgs

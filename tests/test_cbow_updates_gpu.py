@@ -62,7 +62,7 @@ def test_one_warp_makes_the_sequential_update(distger_lib, size, negative, hs):
 
 
 @pytest.mark.parametrize("mode,size,negative", [("cbow", 64, 5), ("cbow", 100, 3), ("cbow", 128, 5), ("sg_shared", 64, 5),
-                                                ("sg_shared", 128, 3), ("sg_shared", 200, 5)])
+                                                ("sg_shared", 128, 3), ("sg_shared", 200, 5), ("sg_shared", 256, 4)])
 def test_two_walks_to_a_warp(distger_lib, mode, size, negative):
     n, length = 6000, 8
     words = np.random.default_rng(4).permutation(n * length).astype(np.uint32)

@@ -56,7 +56,8 @@ def _ratios(corpus, **kw):
 
 
 @pytest.mark.parametrize("size,window,negative,most", [
-    (64, 8, 3, 4), (128, 5, 5, 4), (200, 10, 5, 4), (64, 7, 7, 1.5), (64, 9, 8, 1.5), (256, 5, 7, 1.5), (128, 5, 2, 1.5)])
+    (64, 8, 3, 1.5), (100, 9, 3, 1.5), (128, 5, 5, 1.5), (200, 10, 5, 4), (256, 6, 4, 4), (200, 8, 3, 1.5), (64, 7, 7, 1.5),
+    (64, 9, 8, 1.5), (256, 5, 7, 1.5), (128, 5, 2, 1.5)])
 def test_shared_negatives(corpus, size, window, negative, most):
     assert max(_ratios(corpus, mode="sg_shared", size=size, window=window, negative=negative)) <= most
 

@@ -17,14 +17,15 @@
 // hold two walks each and train two pairs of either in turn.
 //
 // A round of the 50,000-vertex graph at size 200, window 5, negative 5, with its
-// read-back: 21.3 -> 11.9 ms.
+// read-back: 21.2 -> 11.9 ms.  What bounds it now: the L2's reductions, 4.8 TB/s of them,
+// for a lane's eight columns are two 16-byte atomics and each sector is reduced twice.
 //
 // Why 256 columns and four or five negatives.  Each negative row is read once for two
 // pairs, so it misses the updates of more pairs of other walks.  Over the distance of two
 // equal runs of the one-pair kernel from each other (graphs of 10,000 to 200,000
-// vertices), rows of 256 columns with four or five negatives end 0.9 to 1.6 times as far
-// from that kernel's after one pass and 1.0 to 2.5 times after two (its own runs: 1.5 to
-// 2.2).  With three they are up to 2.0 and 2.7 times as far, with seven and eight up to
+// vertices), rows of 256 columns with four or five negatives end 1.0 to 1.6 times as far
+// from that kernel's after one pass and 1.4 to 2.7 times after two (its own runs: 1.3 to
+// 2.5).  With three they are up to 2.0 and 2.7 times as far, with seven and eight up to
 // 1.9.  At 64 and 128 columns, where that kernel has 32 warps an SM and not 16, it is up to
 // 3.0 (64 columns, seven negatives), and single values of the output rows end up to 11
 // times further off than its own runs show, on graphs of 10,000 to 16,000 vertices above

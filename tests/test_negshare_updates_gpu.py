@@ -38,7 +38,7 @@ def _of_the_update(rows, want, init):
 
 
 @pytest.mark.parametrize("negative", [3, 4, 5, 8])
-@pytest.mark.parametrize("size", [64, 65, 100, 128, 200, 256])
+@pytest.mark.parametrize("size", [64, 65, 100, 128, 130, 200, 250, 256])
 def test_one_warp_makes_the_sequential_update(distger_lib, size, negative):
     offs, verts = _stepping_back(10, 16, size)
     counts = np.random.default_rng(1).integers(1, 200, size=V).astype(np.uint32)
